@@ -69,216 +69,543 @@ __global__ void spmv_AT_U_kernel(const uint32_t *__restrict__ rp,
     }
 }
 
-// Long rows inside CG: one warp per row, lanes stride over the entries and the
-// partial sums meet in a shuffle tree (order differs from hilbert's left-to-
-// right sum; the bit-exact kernels above are the ones the map API uses).
-__device__ __forceinline__ double warp_row(const uint32_t *__restrict__ ent, uint32_t b, uint32_t e,
-                                           const double *__restrict__ x, const double *__restrict__ p,
-                                           double beta, const double *pal, int lane) {
-    double acc = 0.0;
-    for (uint32_t k = b + lane; k < e; k += 32) {
-        const uint32_t w = __ldg(ent + k);
-        const uint32_t c = w & kDevColMask;
-        double v = __ldg(x + c);
-        if (p) v = __dadd_rn(v, __dmul_rn(beta, __ldg(p + c)));
-        acc += pal[(w >> 27) & 15u] * v;
-    }
-    return warp_sum(acc);
-}
-
-// One SELL slice per warp: lane l forms row perm[32 s + l] of the operator
-// applied to x (RBP: to r + beta p, formed per operand as in the stored
-// update), summing its entries in stored order (the group flag splits the
-// sum as packed_row does).  Table loads stream (evict first) so the vectors
-// stay in L2.
-template <bool RBP>
-__device__ __forceinline__ double sell_row(const SellOp &S, int64_t sl, int lane,
-                                           const double *__restrict__ x, const double *__restrict__ p,
-                                           double beta, const double *pal, uint32_t &row) {
-    const int64_t pos = sl * 32 + lane;
-    row = __ldcs(S.perm + pos);
-    const int len = __ldcs(S.len + pos);
-    const uint32_t base = __ldcs(S.off + sl) + lane;
-    double acc0 = 0.0, acc1 = 0.0;
-    bool grp = false;
-#pragma unroll 4
-    for (int k = 0; k < len; k++) {
-        const uint32_t w = __ldcs(S.ent + base + 32u * k);
-        const uint32_t c = w & kDevColMask;
-        double xv = __ldg(x + c);
-        if (RBP) xv = __dadd_rn(xv, __dmul_rn(beta, __ldg(p + c)));
-        const double v = __dmul_rn(pal[(w >> 27) & 15u], xv);
-        grp = grp || (w >> 31);
-        if (grp) acc1 = __dadd_rn(acc1, v);
-        else acc0 = __dadd_rn(acc0, v);
-    }
-    return grp ? __dadd_rn(acc0, acc1) : acc0;
-}
-
 // ------------------------------------------------------------------ CG
 // Solves (A A^T) y = rhs with rhs = A(c - z) + mu (b - A x), warm-started from
 // y, in the form CG takes on normal equations: with t = A^T p the step
 // length's denominator p.(A A^T p) is ||t||^2, which the pass that forms t
-// sums as it goes, so the update of y and r joins the pass that forms A t.
-// Two grid barriers per iteration:
-//   1. p_new = r + beta p_old, t = A^T p_new, partial ||t||^2
-//      -> alpha = r.r / ||t||^2
-//   2. per row j of A: q_j = (A t)_j, y_j += alpha p_new_j,
-//      r_j -= alpha q_j, partial r.r  -> beta, convergence
-// The t.t and r.r partials live in separate arrays: a block that has passed
-// one barrier writes its next partial while slower blocks may still be
-// summing the other.  Operator rows of up to kCgLongRow entries are applied
-// from the sliced-ELL copies (one warp per 32-row slice), longer rows by a
-// warp each from the CSR tables; every row of A is in exactly one of the
-// two, so the row update of pass 2 covers every dual index once.
-// 3 CTAs per SM: the gathers are latency-bound and gain more from resident
-// warps than from registers (2 CTAs per SM measured 10-15% slower)
-__global__ void __launch_bounds__(kCgThreads, 3) cg_kernel(CgParams P) {
+// sums as it goes.  Two grid barriers per iteration, each carrying its sum:
+//   1. t = A^T p with p = r + beta p_old formed per operand from the pair
+//      (r, p_old), partial ||t||^2                      -> alpha = r.r / ||t||^2
+//   2. per constraint j: q = (A t)_j, p_j again from its pair, y_j += alpha
+//      p_j, r_j -= alpha q, partial r.r                  -> beta, convergence
+// r and p_old are one 16-byte pair, so an operand costs one gather; p is never
+// read by another row in pass 2, so pass 2 replaces the pair in place.
+//
+// Rounding: products and sums are those of the stored order of each row
+// (separate multiply and add), the dot products those of the virtual CTAs
+// (cg_tables.h): 16 warps with one accumulator per lane, a shuffle tree per
+// warp, one per CTA, one over the CTAs.  The iteration count of a solve hangs
+// on the last bits (the residual meets the tolerance on a plateau), so the
+// order is part of the result; a CTA hosts V virtual CTAs, and NW warps share
+// their 16 V virtual warps.
+//
+// What bounds it: dependent loads (entry, then operand) and the two barriers,
+// with all tables and vectors in L2; so a warp has several slices' loads in
+// flight, and one CTA per SM meets at the barrier.
+
+// the operand p (PAIR: r + beta p_old of a pair; else a plain vector)
+template <bool PAIR>
+struct Operand {
+    const double2 *rp;
+    const double *x;
+    double beta;
+    __device__ __forceinline__ double operator()(uint32_t pos) const {
+        if (!PAIR) return x[pos];
+        const double2 v = rp[pos];
+        return __dadd_rn(v.x, __dmul_rn(beta, v.y));
+    }
+};
+
+// a compile-time count
+template <int K>
+struct Count {
+    __device__ constexpr operator int() const { return K; }
+};
+// table words in shared memory, or streamed through L2 without displacing the
+// vectors
+template <bool SMEM>
+struct Words {
+    const uint32_t *p;
+    __device__ __forceinline__ uint32_t operator[](uint32_t k) const { return SMEM ? p[k] : __ldcs(p + k); }
+    __device__ __forceinline__ Words operator+(uint32_t k) const { return Words{p + k}; }
+};
+
+// the lane's row of one slice: entries in stored order, separate multiply and
+// add, flagged entries in a second sum; STEP operands in flight (the loads are
+// unconditional, from position 0 past a row's end, so that none waits for
+// another).  SELF: entries at kCgSelf take coef * self instead.
+template <int STEP, bool SELF, bool SMEM, class X>
+__device__ __forceinline__ double sell_row(const Words<SMEM> &ent, uint32_t width, uint32_t len, const X &x, double self,
+                                           const double *pal) {
+    double acc0 = 0.0, acc1 = 0.0;
+    bool grp = false;
+    for (uint32_t k0 = 0; k0 < width; k0 += STEP) {
+        uint32_t w[STEP];
+        double v[STEP];
+#pragma unroll
+        for (int k = 0; k < STEP; k++) w[k] = k0 + k < len ? ent[32u * (k0 + k)] : 0u;
+#pragma unroll
+        for (int k = 0; k < STEP; k++) {
+            const uint32_t c = w[k] & kDevColMask;
+            v[k] = x(SELF && c == kCgSelf ? 0u : c);
+        }
+#pragma unroll
+        for (int k = 0; k < STEP; k++) {
+            const double cf = pal[(w[k] >> 27) & 15u];
+            const double u = __dmul_rn(cf, SELF && (w[k] & kDevColMask) == kCgSelf ? __dmul_rn(cf, self) : v[k]);
+            const bool in = k0 + k < len;
+            grp = grp || (in && (w[k] >> 31));
+            const double s0 = __dadd_rn(acc0, u), s1 = __dadd_rn(acc1, u);
+            acc0 = in && !grp ? s0 : acc0;
+            acc1 = in && grp ? s1 : acc1;
+        }
+    }
+    return grp ? __dadd_rn(acc0, acc1) : acc0;
+}
+// a long row by one warp: the lanes stride over the entries, a shuffle tree
+template <class X>
+__device__ __forceinline__ double warp_row(const uint32_t *ent, uint32_t b, uint32_t e, const X &x, const double *pal,
+                                           int lane) {
+    double acc = 0.0;
+    for (uint32_t k0 = b; k0 < e; k0 += 128) {
+        uint32_t w[4];
+        double v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = k0 + 32u * k + lane < e ? ent[k0 + 32u * k + lane] : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = x(w[k] & kDevColMask);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (k0 + 32u * k + lane < e) acc += pal[(w[k] >> 27) & 15u] * v[k];
+    }
+    return warp_sum(acc);
+}
+
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// V virtual CTAs to a CTA of NW warps; U plain slices and STEP operands of
+// another row in flight.  A virtual warp's tables (a few KB) are always read
+// from shared memory: a table word read from L2 would put one more dependent
+// load before every operand (12 joint rings: 24 us per iteration against 40).
+// Where the SM holds both passes' tables they are copied once (kCgBoth); else
+// the two passes share the region, and each warp starts the copy of the next
+// pass's tables as it ends a pass, so that it runs behind the barrier
+// (kCgOneRegion); tables too large for that are streamed from L2 and HBM
+// (kCgStreamed: evict first, the vectors stay in L2).
+template <int NW, int V, int U, int STEP, int CTAS, CgTablesIn IN>
+__global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
+    constexpr int VW = kCgVirtualWarps * V;    // virtual warps of a full CTA
+    constexpr int H = VW / NW;                 // per warp
+    constexpr bool SMEM = IN != kCgStreamed, SHARED = IN == kCgOneRegion;
+    static_assert(H * NW == VW, "whole virtual warps");
+    extern __shared__ __align__(16) uint32_t cg_sm[];
     __shared__ double palA[16], palT[16];
-    __shared__ double red[32];
-    __shared__ double bcast;
-    __shared__ int flag;
+    __shared__ double red[VW], total;
+    __shared__ int fail;
     __shared__ unsigned long long tmark;   // phase clock (CTA 0, thread 0)
-    if (threadIdx.x < 16) {
-        palA[threadIdx.x] = P.palA.v[threadIdx.x];
-        palT[threadIdx.x] = P.palT.v[threadIdx.x];
+    __shared__ uint32_t hostA[V], hostT[V];
+    // per virtual warp and side: first and past-last slice, where the tables
+    // stand in cg_sm (off: word of slice b; ent: word of entry 0; len: byte of
+    // slice b)
+    struct Run {
+        uint32_t b, e, gw, off, ent, len;
+    };
+    __shared__ Run runA[VW], runT[VW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cta = blockIdx.x;
+    if (tid < 16) {
+        palA[tid] = P.palA.v[tid];
+        palT[tid] = P.palT.v[tid];
+    }
+    if (tid == 0) fail = 0;
+    if (tid < V) {
+        hostA[tid] = P.dual.host[cta * V + tid];
+        hostT[tid] = P.prim.host[cta * V + tid];
+    }
+    const uint32_t all = (uint32_t)P.nvirtual * kCgVirtualWarps;
+    __syncthreads();
+    auto words = [&](const CgRows &R, const Run &r) {
+        return r.gw == 0xffffffffu ? 0u
+                                   : cg_table_words(r.e - r.b, (R.off[r.e] & ~kCgPlain) - (R.off[r.b] & ~kCgPlain));
+    };
+    if (tid < VW) {
+        auto init = [&](Run &r, const CgRows &R, uint32_t vc) {
+            r = Run{0u, 0u, 0xffffffffu, 0u, 0u, 0u};
+            if (vc == 0xffffffffu) return;
+            r.gw = vc * kCgVirtualWarps + tid % kCgVirtualWarps;
+            r.b = R.split[r.gw];
+            r.e = R.split[r.gw + 1];
+        };
+        init(runA[tid], P.dual, hostA[tid / kCgVirtualWarps]);
+        init(runT[tid], P.prim, hostT[tid / kCgVirtualWarps]);
+        runA[tid].off = words(P.dual, runA[tid]);
+        runT[tid].off = words(P.prim, runT[tid]);
     }
     __syncthreads();
-    // 32-bit thread indices (a grid holds far fewer than 2^31 threads);
-    // the kernel runs at the 40-register limit of 3 CTAs per SM
-    const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned stride = gridDim.x * blockDim.x;
-    const int nb = gridDim.x;
-
-    const int lane = threadIdx.x & 31;
-    const unsigned gwarp = gtid >> 5, nwarps = stride >> 5;
-    // optional phase clock: CTA 0 adds the time from barrier to barrier
-    if (gtid == 0) tmark = global_ns();
-    auto lap = [&](int k) {
-        if (P.phase_ns != nullptr && gtid == 0) {
+    if (SMEM && tid == 0) {   // where each run's tables go
+        uint32_t at = 0;
+        for (int w = 0; w < VW; w++) {
+            const uint32_t na = runA[w].off, nt = runT[w].off;
+            runA[w].ent = at;
+            runT[w].ent = SHARED ? at : at + na;
+            at += SHARED ? max(na, nt) : na + nt;
+        }
+    }
+    __syncthreads();
+    // start the copy of a run's tables: entries, lengths, offsets
+    auto fetch = [&](const CgRows &R, const Run &r) {
+        if (r.gw == 0xffffffffu) return;
+        const uint32_t e0 = R.off[r.b] & ~kCgPlain, ne = (R.off[r.e] & ~kCgPlain) - e0, n = r.e - r.b;
+        const uint32_t at = r.ent + e0;   // r.ent is the word of entry 0 (below)
+        for (uint32_t k = 4u * lane; k < ne; k += 128u) cp_async16(cg_sm + at + k, R.ent + e0 + k);
+        for (uint32_t k = lane; k < 2u * n; k += 32u)
+            cp_async16((uint8_t *)cg_sm + r.len + 16u * k, R.len + 32u * (size_t)r.b + 16u * k);
+        for (uint32_t k = lane; k <= n; k += 32u) cp_async4(cg_sm + r.off + k, R.off + r.b + k);
+    };
+    if (SMEM && tid < VW) {
+        auto place = [&](Run &r, const CgRows &R) {
+            if (r.gw == 0xffffffffu) return;
+            const uint32_t e0 = R.off[r.b] & ~kCgPlain, ne = (R.off[r.e] & ~kCgPlain) - e0, at = r.ent;
+            r.ent = at - e0;
+            r.len = 4u * (at + ne);
+            r.off = at + ne + 8u * (r.e - r.b);
+        };
+        place(runA[tid], P.dual);
+        place(runT[tid], P.prim);
+    }
+    const uint32_t dl = 32u * P.dual.nslices, tl = 32u * P.prim.nslices;   // positions of the long rows
+    GridSum bar{P.slots, P.nvirtual, P.count, P.status, P.spin_limit, &total, &fail, 0u};
+    // barrier + sum of one value per lane of every virtual warp
+    auto sync = [&](const double (&loc)[H], const uint32_t *host, double &sum) {
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const double w = warp_sum(loc[h]);
+            if (lane == 0) red[warp + h * NW] = w;
+        }
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                double s = lane < kCgVirtualWarps ? red[v * kCgVirtualWarps + lane] : 0.0;
+                s = warp_sum(s);
+                if (lane == 0 && host[v] != 0xffffffffu) __stcg(bar.set() + host[v], s);
+            }
+            bar.arrive_and_sum(lane);
+        }
+        __syncthreads();
+        return bar.done(sum);
+    };
+    if (tid == 0) tmark = global_ns();
+    __syncthreads();
+    // tables of the pass ahead (SHARED), or of both passes once
+    auto fetch_T = [&](bool start) {
+        if (!SMEM || (!SHARED && !start)) return;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < H; h++) fetch(P.prim, runT[warp + h * NW]);
+    };
+    auto fetch_A = [&](bool start) {
+        if (!SMEM || (!SHARED && !start)) return;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < H; h++) fetch(P.dual, runA[warp + h * NW]);
+    };
+    auto fetched = [&]() {
+        if (!SMEM) return;
+        cp_async_wait_all();
+        __syncwarp();
+    };
+    fetch_T(true);
+    if (!SHARED) fetch_A(true);
+    auto lap = [&](int k) {   // optional phase clock: CTA 0 adds the time from barrier to barrier
+        if (P.phase_ns != nullptr && cta == 0 && tid == 0) {
             const unsigned long long now = global_ns();
             P.phase_ns[k] += now - tmark;
             tmark = now;
         }
     };
+    // t = A^T x over a run's slices: stored except at singles, squares into
+    // loc in order (loc null: no squares)
+    auto apply_T = [&](const Run &r, const auto &x, double *loc) {
+        const uint32_t e = r.e;
+        const Words<SMEM> ent{SMEM ? cg_sm + r.ent + lane : P.prim.ent + lane};
+        const Words<SMEM> off{SMEM ? cg_sm + r.off - r.b : P.prim.off};
+        const uint8_t *len = SMEM ? (const uint8_t *)cg_sm + r.len - 32 * (size_t)r.b + lane : P.prim.len + lane;
+        // K plain slices from s on
+        auto plain = [&](auto K, const uint32_t *o) {
+            uint32_t w[K];
+            double v[K];
+#pragma unroll
+            for (int u = 0; u < K; u++) w[u] = ent[o[u] & ~kCgPlain];
+#pragma unroll
+            for (int u = 0; u < K; u++) v[u] = x(w[u] & kDevColMask);
+            if (loc)
+#pragma unroll
+                for (int u = 0; u < K; u++) {
+                    const double tv = __dmul_rn(palT[w[u] >> 27], v[u]);
+                    *loc = fma(tv, tv, *loc);
+                }
+        };
+        for (uint32_t s = r.b; s < e;) {
+            uint32_t o[U];
+            bool all_plain = s + U <= e;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                o[u] = off[min(s + u, e)];
+                all_plain = all_plain && (o[u] & kCgPlain);
+            }
+            if (all_plain) {
+                plain(Count<U>(), o);
+                s += U;
+                continue;
+            }
+            if (o[0] & kCgPlain) {
+                plain(Count<1>(), o);
+                s++;
+                continue;
+            }
+            const uint32_t n = len[32u * s], o1 = off[s + 1] & ~kCgPlain, width = (o1 - o[0]) >> 5;
+            if (n != kCgPadding) {
+                const double tv = width <= 2 ? sell_row<2, false, SMEM>(ent + o[0], width, n & 0x7fu, x, 0.0, palT)
+                                             : sell_row<STEP, false, SMEM>(ent + o[0], width, n & 0x7fu, x, 0.0, palT);
+                if (!(n & kCgSingle)) P.t[32u * s + lane] = tv;
+                if (loc) *loc = fma(tv, tv, *loc);
+            }
+            s++;
+        }
+    };
+    auto long_T = [&](uint32_t gw, const auto &x, double *loc) {
+        for (uint32_t l = gw; l < P.prim.nlong; l += all) {
+            const double v = warp_row(P.prim.lent, P.prim.lrp[l], P.prim.lrp[l + 1], x, palT, lane);
+            if (lane == 0) {
+                P.t[tl + l] = v;
+                if (loc) *loc = fma(v, v, *loc);
+            }
+        }
+    };
+    // f(position, (A t) there, own) over a run's slices, in order; own =
+    // own0(position) is loaded with the entries, self(own) is the p that the
+    // row's singles take
+    const Operand<false> tx{nullptr, P.t, 0.0};
+    auto apply_A = [&](const Run &r, auto &&own0, auto &&self, auto &&f) {
+        const uint32_t e = r.e;
+        const Words<SMEM> ent{SMEM ? cg_sm + r.ent + lane : P.dual.ent + lane};
+        const Words<SMEM> off{SMEM ? cg_sm + r.off - r.b : P.dual.off};
+        const uint8_t *len = SMEM ? (const uint8_t *)cg_sm + r.len - 32 * (size_t)r.b + lane : P.dual.len + lane;
+        auto plain = [&](auto K, uint32_t s, const uint32_t *o) {
+            uint32_t w[K][2];
+            double v[K][2];
+            decltype(own0(0u)) own[K];
+#pragma unroll
+            for (int u = 0; u < K; u++) {
+                own[u] = own0(32u * (s + u) + lane);
+                w[u][0] = ent[o[u] & ~kCgPlain];
+                w[u][1] = ent[(o[u] & ~kCgPlain) + 32u];
+            }
+#pragma unroll
+            for (int u = 0; u < K; u++)
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const uint32_t c = w[u][k] & kDevColMask;
+                    v[u][k] = P.t[c == kCgSelf ? 0u : c];
+                }
+#pragma unroll
+            for (int u = 0; u < K; u++) {
+                const double sv = self(own[u]);
+                double q[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const double c = palA[w[u][k] >> 27];
+                    q[k] = __dmul_rn(c, (w[u][k] & kDevColMask) == kCgSelf ? __dmul_rn(c, sv) : v[u][k]);
+                }
+                f(32u * (s + u) + lane, __dadd_rn(q[0], q[1]), own[u]);
+            }
+        };
+        for (uint32_t s = r.b; s < e;) {
+            uint32_t o[U];
+            bool all_plain = s + U <= e;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                o[u] = off[min(s + u, e)];
+                all_plain = all_plain && (o[u] & kCgPlain);
+            }
+            if (all_plain) {
+                plain(Count<U>(), s, o);
+                s += U;
+                continue;
+            }
+            if (o[0] & kCgPlain) {
+                plain(Count<1>(), s, o);
+                s++;
+                continue;
+            }
+            const uint32_t n = len[32u * s], o1 = off[s + 1] & ~kCgPlain, width = (o1 - o[0]) >> 5;
+            if (n != kCgPadding) {
+                const auto own = own0(32u * s + lane);
+                const double q = width <= 2 ? sell_row<2, true, SMEM>(ent + o[0], width, n, tx, self(own), palA)
+                                            : sell_row<(STEP < 8 ? STEP : 8), true, SMEM>(ent + o[0], width, n, tx,
+                                                                                          self(own), palA);
+                f(32u * s + lane, q, own);
+            }
+            s++;
+        }
+    };
+    auto long_A = [&](uint32_t gw, auto &&own0, auto &&f) {
+        for (uint32_t l = gw; l < P.dual.nlong; l += all) {
+            const double v = warp_row(P.dual.lent, P.dual.lrp[l], P.dual.lrp[l + 1], tx, palA, lane);
+            if (lane == 0) f(dl + l, v, own0(dl + l));
+        }
+    };
+    // copy(original row, position) over the own constraints, C at a time
+    constexpr int C = 4;
+    auto own_rows = [&](auto &&load, auto &&store) {
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const Run &r = runA[warp + h * NW];
+            if (r.gw == 0xffffffffu) continue;
+            for (uint32_t s = r.b; s < r.e; s += C) {
+                uint32_t o[C];
+                double v[C];
+#pragma unroll
+                for (int u = 0; u < C; u++) o[u] = s + u < r.e ? P.orig[32u * (s + u) + lane] : 0xffffffffu;
+#pragma unroll
+                for (int u = 0; u < C; u++) v[u] = o[u] != 0xffffffffu ? load(o[u], 32u * (s + u) + lane) : 0.0;
+#pragma unroll
+                for (int u = 0; u < C; u++)
+                    if (o[u] != 0xffffffffu) store(o[u], 32u * (s + u) + lane, v[u]);
+            }
+            if (lane == 0)
+                for (uint32_t l = r.gw; l < P.dual.nlong; l += all)
+                    store(P.orig[dl + l], dl + l, load(P.orig[dl + l], dl + l));
+        }
+    };
 
     // r = rhs - A A^T y
-    for (int64_t sl = P.st.split[gwarp], se = P.st.split[gwarp + 1]; sl < se; sl++) {
-        uint32_t row;
-        const double v = sell_row<false>(P.st, sl, lane, P.y, nullptr, 0.0, palT, row);
-        if (row != 0xffffffffu) P.t[row] = v;
-    }
-    for (int64_t w = gwarp; w < P.n_long_t; w += nwarps) {
-        const int64_t i = __ldg(P.long_t + w);
-        const double v = warp_row(P.t_ent, __ldg(P.t_rp + i), __ldg(P.t_rp + i + 1), P.y, nullptr, 0.0,
-                                  palT, lane);
-        if (lane == 0) P.t[i] = v;
-    }
-    if (!grid_sync(P.bar, P.status, P.spin_limit, &flag)) return;
-    double loc = 0.0;
-    for (int64_t sl = P.sa.split[gwarp], se = P.sa.split[gwarp + 1]; sl < se; sl++) {
-        uint32_t row;
-        const double av = sell_row<false>(P.sa, sl, lane, P.t, nullptr, 0.0, palA, row);
-        if (row != 0xffffffffu) {
-            const double v = P.Acz[row] + P.mu * (P.b[row] - P.Ax[row]) - av;
-            P.r[row] = v;
-            loc += v * v;
+    double zero[H] = {}, loc[H], sum, rs;
+    own_rows([&](uint32_t o, uint32_t) { return P.y[o]; }, [&](uint32_t, uint32_t j, double v) { P.yp[j] = v; });
+    auto stopped = [&]() {   // no copy may be in flight when a CTA leaves
+        cp_async_wait_all();
+    };
+    if (!sync(zero, hostA, sum)) return stopped();
+    fetched();
+    {
+        const Operand<false> yx{nullptr, P.yp, 0.0};
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const Run &r = runT[warp + h * NW];
+            if (r.gw == 0xffffffffu) continue;
+            apply_T(r, yx, nullptr);
+            long_T(r.gw, yx, nullptr);
         }
     }
-    for (int64_t w = gwarp; w < P.n_long_a; w += nwarps) {
-        const int64_t j = __ldg(P.long_a + w);
-        const double av = warp_row(P.a_ent, __ldg(P.a_rp + j), __ldg(P.a_rp + j + 1), P.t, nullptr, 0.0,
-                                   palA, lane);
-        if (lane == 0) {
-            const double v = P.Acz[j] + P.mu * (P.b[j] - P.Ax[j]) - av;
-            P.r[j] = v;
-            loc += v * v;
+    fetch_A(false);
+    if (!sync(zero, hostA, sum)) return stopped();
+    fetched();
+    {
+        struct Own {
+            double y, acz, b, ax;
+        };
+        auto own0 = [&](uint32_t j) {
+            const uint32_t o = P.orig[j];
+            return Own{P.yp[j], P.Acz[o], P.b[o], P.Ax[o]};
+        };
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            loc[h] = 0.0;
+            const Run &r = runA[warp + h * NW];
+            if (r.gw == 0xffffffffu) continue;
+            auto f = [&](uint32_t j, double av, const Own &o) {
+                const double v = o.acz + P.mu * (o.b - o.ax) - av;
+                P.rp[j] = make_double2(v, 0.0);
+                loc[h] = fma(v, v, loc[h]);
+            };
+            apply_A(r, own0, [](const Own &o) { return o.y; }, f);
+            long_A(r.gw, own0, f);
         }
     }
-    double s = block_sum(loc, red);
-    if (threadIdx.x == 0) P.partials[nb + blockIdx.x] = s;
-    if (!grid_sync(P.bar, P.status, P.spin_limit, &flag)) return;
+    fetch_T(false);
+    if (!sync(loc, hostA, rs)) return stopped();
     lap(0);
-    double rs = sum_partials(P.partials + nb, nb, &bcast);
 
     int it = 0;
     double beta = 0.0;
-    // p_old is r on the first iteration (beta = 0), then p0 and p1 alternate
-    // as p_new and p_old
     bool done = !(sqrt(rs) >= P.tol);
     while (!done && it < P.maxit) {
-        // pass 1: t = A^T (r + beta p_old), ||t||^2; p_new = r + beta p_old
-        const double *pold = it == 0 ? P.r : ((it & 1) ? P.p0 : P.p1);
-        double *pnew = (it & 1) ? P.p1 : P.p0;
-        loc = 0.0;
-        for (int64_t sl = P.st.split[gwarp], se = P.st.split[gwarp + 1]; sl < se; sl++) {
-            uint32_t row;
-            const double v = sell_row<true>(P.st, sl, lane, P.r, pold, beta, palT, row);
-            if (row != 0xffffffffu) {
-                P.t[row] = v;
-                loc += v * v;
-            }
+        // pass 1
+        fetched();
+        const Operand<true> px{P.rp, nullptr, beta};
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            loc[h] = 0.0;
+            const Run &r = runT[warp + h * NW];
+            if (r.gw == 0xffffffffu) continue;
+            apply_T(r, px, &loc[h]);
+            long_T(r.gw, px, &loc[h]);
         }
-        for (int64_t w = gwarp; w < P.n_long_t; w += nwarps) {
-            const int64_t i = __ldg(P.long_t + w);
-            const double v = warp_row(P.t_ent, __ldg(P.t_rp + i), __ldg(P.t_rp + i + 1), P.r, pold,
-                                      beta, palT, lane);
-            if (lane == 0) {
-                P.t[i] = v;
-                loc += v * v;
-            }
-        }
-        for (int64_t j = gtid; j < P.nd; j += stride)
-            pnew[j] = __dadd_rn(P.r[j], __dmul_rn(beta, pold[j]));
-        s = block_sum(loc, red);
-        if (threadIdx.x == 0) P.partials[blockIdx.x] = s;
-        if (!grid_sync(P.bar, P.status, P.spin_limit, &flag)) return;
+        fetch_A(false);
+        double tt;
+        if (!sync(loc, hostT, tt)) break;
         lap(1);
-        const double tt = sum_partials(P.partials, nb, &bcast);
         if (!(tt > 0.0)) break;   // range of A A^T exhausted (or non-finite)
         const double alpha = rs / tt;
 
-        // pass 2: q = A t row by row, y += alpha p_new, r -= alpha q, r.r
-        loc = 0.0;
-        for (int64_t w = gwarp; w < P.n_long_a; w += nwarps) {
-            const int64_t j = __ldg(P.long_a + w);
-            const double q = warp_row(P.a_ent, __ldg(P.a_rp + j), __ldg(P.a_rp + j + 1), P.t, nullptr,
-                                      0.0, palA, lane);
-            if (lane == 0) {
-                P.y[j] += alpha * pnew[j];
-                const double rv = P.r[j] - alpha * q;
-                P.r[j] = rv;
-                loc += rv * rv;
-            }
+        // pass 2
+        fetched();
+        struct Own {
+            double2 rp;
+            double y;
+        };
+        auto own0 = [&](uint32_t j) { return Own{P.rp[j], P.yp[j]}; };
+        auto dir = [&](const Own &o) { return __dadd_rn(o.rp.x, __dmul_rn(beta, o.rp.y)); };
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            loc[h] = 0.0;
+            const Run &r = runA[warp + h * NW];
+            if (r.gw == 0xffffffffu) continue;
+            auto f = [&](uint32_t j, double q, const Own &o) {
+                const double pn = dir(o);
+                P.yp[j] = fma(alpha, pn, o.y);
+                const double rv = fma(-alpha, q, o.rp.x);
+                P.rp[j] = make_double2(rv, pn);
+                loc[h] = fma(rv, rv, loc[h]);
+            };
+            long_A(r.gw, own0, f);
+            apply_A(r, own0, dir, f);
         }
-        for (int64_t sl = P.sa.split[gwarp], se = P.sa.split[gwarp + 1]; sl < se; sl++) {
-            uint32_t row;
-            const double q = sell_row<false>(P.sa, sl, lane, P.t, nullptr, 0.0, palA, row);
-            if (row != 0xffffffffu) {
-                P.y[row] += alpha * pnew[row];
-                const double rv = P.r[row] - alpha * q;
-                P.r[row] = rv;
-                loc += rv * rv;
-            }
-        }
-        s = block_sum(loc, red);
-        if (threadIdx.x == 0) P.partials[nb + blockIdx.x] = s;
-        if (!grid_sync(P.bar, P.status, P.spin_limit, &flag)) return;
+        fetch_T(false);
+        double rs_new;
+        if (!sync(loc, hostA, rs_new)) break;
         lap(2);
-        const double rs_new = sum_partials(P.partials + nb, nb, &bcast);
         it++;
         if (!(rs_new == rs_new)) {   // NaN
-            if (gtid == 0) atomicExch(P.status, kStatusNan);
+            if (cta == 0 && tid == 0) atomicExch(P.status, kStatusNan);
             break;
         }
         done = sqrt(rs_new) < P.tol;
         beta = rs_new / rs;
         rs = rs_new;
     }
-    if (gtid == 0) {
+    cp_async_wait_all();   // the tables of a pass that does not come
+    if (fail) return;
+    own_rows([&](uint32_t, uint32_t j) { return P.yp[j]; }, [&](uint32_t o, uint32_t, double v) { P.y[o] = v; });
+    if (cta == 0 && tid == 0) {
         P.out[0] = (double)it;
         P.out[1] = sqrt(rs);
     }
+}
+
+// Measured on B200 (us per CG iteration; in brackets the former kernel: two
+// gathers per operand, tables read from L2, three CTAs of 512 threads per SM,
+// a barrier of three round trips):
+//   6-site ring 7.4 (22.9), (9e,9o) 11.5 (30), (6e,6o) DQGT2 12.9 (31),
+//   DOCI (10e,10o) 6.6 (15.9), 12 joint rings 18.1 (48), (20e,20o) 47 (84).
+// Warps and operands in flight, same order: a warp per virtual warp where one
+// or two virtual CTAs share an SM ((9e,9o), 16 warps: 12.0); three on 24 warps
+// (on 16 warps (20e,20o) took 53, as three CTAs of 16 warps 64).
+CgShape cg_shape(int v, CgTablesIn in) {
+    if (in == kCgStreamed) return {(const void *)cg_kernel<16, 1, 2, 4, 3, kCgStreamed>, 512};
+    if (v == 1) return {(const void *)cg_kernel<16, 1, 1, 8, 1, kCgBoth>, 512};
+    if (v == 2) return {(const void *)cg_kernel<32, 2, 1, 8, 1, kCgBoth>, 1024};
+    if (in == kCgBoth) return {(const void *)cg_kernel<24, 3, 2, 8, 1, kCgBoth>, 768};
+    return {(const void *)cg_kernel<24, 3, 2, 4, 1, kCgOneRegion>, 768};
 }
 
 // ------------------------------------------------------- CG start

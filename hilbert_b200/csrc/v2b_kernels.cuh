@@ -4,26 +4,17 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "cg_tables.h"
 #include "v2b_device.cuh"
 
 namespace v2b {
 
 constexpr int kSpmvThreads = 256;
-constexpr int kCgThreads = 512;
-constexpr uint32_t kCgLongRow = 32;   // rows with more entries get a whole warp inside CG
-
-// Sliced ELL copy of an operator for the CG kernel (SELL-C-sigma, C = 32):
-// rows of at most kCgLongRow entries, sorted by length inside windows of
-// kSellSigma rows, in slices of 32 rows stored column-major (entry k of the
-// slice's lane l at off[s] + 32 k + l), perm = original row (0xffffffff on
-// padding lanes), len = its entry count.  A warp handles a slice: its loads
-// are coalesced and independent of one another.
-constexpr int kSellSigma = 8192;
-struct SellOp {
-    const uint32_t *ent, *perm, *off;
+// One side of the constraint operator as the CG kernel reads it (cg_tables.h)
+struct CgRows {
+    const uint32_t *off, *ent, *lrp, *lent, *split, *host;
     const uint8_t *len;
-    int64_t nslices;
-    const uint32_t *split;   // CG warp w takes slices split[w] .. split[w + 1] - 1
+    uint32_t nslices, nlong;
 };
 constexpr int kJacobiThreads = 512;
 constexpr int kJacobiMaxDim = 160;     // np*np doubles + rotations must fit in 227 KB
@@ -34,26 +25,40 @@ struct Palette {
 };
 
 struct CgParams {
-    const uint32_t *a_rp, *a_ent;   // A   (rows = dual constraints)
-    const uint32_t *t_rp, *t_ent;   // A^T (rows = primal variables)
-    const int64_t *long_a, *long_t; // rows longer than kCgLongRow (warp per row)
-    int64_t n_long_a, n_long_t;
-    SellOp sa, st;                  // the other rows of A and A^T
+    CgRows dual, prim;              // A by constraint, A^T by primal variable
+    const uint32_t *orig;           // original row of each dual position
     Palette palA, palT;
-    int64_t np, nd;
-    const double *Ax, *Acz, *b;     // rhs = Acz + mu (b - Ax)
+    const double *Ax, *Acz, *b;     // rhs = Acz + mu (b - Ax), original order
     double mu;
-    double *y, *r, *p0, *p1, *t;
-    double *partials;               // >= 2 * gridDim.x (t.t partials, then r.r partials)
-    GridBarrier *bar;
+    double *y;                      // original order, in / out
+    double2 *rp;                    // by dual position: the residual and the last direction
+    double *yp, *t;                 // by dual and by primal position
+    double *slots;                  // 2 x virtual CTAs
+    unsigned int *count;            // 0 before the launch
     int *status;
     long long spin_limit;
     double tol;
     int maxit;
+    int nvirtual;                   // virtual CTAs, the dot products' partial sums
     double *out;                    // out[0] = iterations, out[1] = final ||r||
     unsigned long long *phase_ns;   // null, or 4 sums of ns: initial residual, pass 1 (A^T p),
                                     // pass 2 (A t and the update), and a slot left at zero
 };
+// where the CG kernel reads its tables: shared memory, both passes' side by
+// side or in turn in one region, or global memory
+enum CgTablesIn { kCgBoth, kCgOneRegion, kCgStreamed };
+// The CG kernel for v = 1, 2 or 3 virtual CTAs to a CTA, one CTA per SM
+// (kCgStreamed: v = 1, three CTAs per SM), and its thread count
+struct CgShape {
+    const void *kernel;
+    int threads;
+};
+CgShape cg_shape(int v, CgTablesIn in);
+// shared-memory words of one virtual warp's tables: slices, their entries
+__host__ __device__ inline uint32_t cg_table_words(uint32_t nslices, uint32_t nent) {
+    return nent + 8u * nslices + ((nslices + 4u) & ~3u);
+}
+constexpr size_t kCgStaticSmem = 4096;   // at least the kernel's static shared memory
 
 __global__ void spmv_kernel(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ent,
                             int64_t nrows, const double *__restrict__ x, double *__restrict__ y,
@@ -67,7 +72,6 @@ __global__ void spmv_AT_U_kernel(const uint32_t *__restrict__ rp,
                                  const double *__restrict__ y, const double *__restrict__ x,
                                  const double *__restrict__ c, double mu,
                                  double *__restrict__ ATy, double *__restrict__ U, Palette pal);
-__global__ void cg_kernel(CgParams P);
 // the CG starting point of the next outer iteration from the last dual
 // solutions (order 0: y itself, 1: 2y - y1, 2: 3y - 3y1 + y2); y1, y2 shift
 __global__ void extrapolate_y_kernel(double *__restrict__ y, double *__restrict__ y1,

@@ -27,6 +27,7 @@
 #include "v2b_kernels.cuh"
 #include "v2b_orbital.cuh"
 #include "v2b_refine.cuh"
+#include "cg_tables.h"
 #include "v2rdm_b200.h"
 #include "v2rdm_problem.h"
 #include "rdm_records.h"
@@ -99,16 +100,9 @@ void ensure_device() {
 
 struct DeviceOp {
     uint32_t *rp = nullptr, *ent = nullptr;
-    int64_t *long_rows = nullptr;   // rows longer than kCgLongRow
-    int64_t nrows = 0, n_long = 0;
+    int64_t nrows = 0;
     size_t nnz = 0;
     v2b::Palette pal{};
-    // sliced-ELL copy of the other rows, for the CG kernel
-    uint32_t *sell_ent = nullptr, *sell_perm = nullptr, *sell_off = nullptr;
-    uint8_t *sell_len = nullptr;
-    int64_t nslices = 0;
-    std::vector<uint32_t> host_off;   // slice offsets (entries), for the work split
-    uint32_t *sell_split = nullptr;   // per CG warp: its first slice (nwarps + 1 entries)
 
     void upload(const v2b::PackedOperator &op) {
         nrows = op.nrows;
@@ -118,122 +112,110 @@ struct DeviceOp {
         V2B_CK(cudaMemcpy(rp, op.row_ptr.data(), op.row_ptr.size() * 4, cudaMemcpyHostToDevice));
         V2B_CK(cudaMemcpy(ent, op.entries.data(), nnz * 4, cudaMemcpyHostToDevice));
         for (int i = 0; i < 16; i++) pal.v[i] = i < (int)op.palette.size() ? op.palette[i] : 0.0;
-        std::vector<int64_t> lr;
-        for (int64_t r = 0; r < nrows; r++)
-            if (op.row_ptr[r + 1] - op.row_ptr[r] > v2b::kCgLongRow) lr.push_back(r);
-        n_long = (int64_t)lr.size();
-        long_rows = dalloc<int64_t>(lr.size());
-        if (n_long) V2B_CK(cudaMemcpy(long_rows, lr.data(), lr.size() * 8, cudaMemcpyHostToDevice));
-        build_sell(op);
-    }
-
-    // SELL-C-sigma with C = 32: inside each window of kSellSigma rows the
-    // short rows are sorted by length (longest first, stable), cut into
-    // slices of 32 (the window's last slice padded with empty lanes) and
-    // stored column-major at the slice's width
-    void build_sell(const v2b::PackedOperator &op) {
-        std::vector<uint32_t> e, perm, off;
-        std::vector<uint8_t> len;
-        std::vector<std::pair<uint32_t, uint32_t>> w;   // (length, row)
-        for (int64_t w0 = 0; w0 < nrows; w0 += v2b::kSellSigma) {
-            const int64_t w1 = std::min<int64_t>(nrows, w0 + v2b::kSellSigma);
-            w.clear();
-            for (int64_t r = w0; r < w1; r++) {
-                const uint32_t L = op.row_ptr[r + 1] - op.row_ptr[r];
-                if (L <= v2b::kCgLongRow) w.push_back({L, (uint32_t)r});
-            }
-            std::stable_sort(w.begin(), w.end(), [](const std::pair<uint32_t, uint32_t> &a,
-                                                    const std::pair<uint32_t, uint32_t> &b) {
-                return a.first > b.first;
-            });
-            for (size_t s0 = 0; s0 < w.size(); s0 += 32) {
-                const size_t cnt = std::min<size_t>(32, w.size() - s0);
-                const uint32_t width = w[s0].first;
-                off.push_back((uint32_t)e.size());
-                for (uint32_t k = 0; k < width; k++)
-                    for (size_t l = 0; l < 32; l++) {
-                        uint32_t v = 0;
-                        if (l < cnt && k < w[s0 + l].first) v = op.entries[op.row_ptr[w[s0 + l].second] + k];
-                        e.push_back(v);
-                    }
-                for (size_t l = 0; l < 32; l++) {
-                    perm.push_back(l < cnt ? w[s0 + l].second : 0xffffffffu);
-                    len.push_back(l < cnt ? (uint8_t)w[s0 + l].first : 0);
-                }
-            }
-        }
-        nslices = (int64_t)off.size();
-        off.push_back((uint32_t)e.size());
-        host_off = off;
-        sell_ent = dalloc<uint32_t>(e.size());
-        sell_perm = dalloc<uint32_t>(perm.size());
-        sell_len = dalloc<uint8_t>(len.size());
-        sell_off = dalloc<uint32_t>(off.size());
-        if (!e.empty()) V2B_CK(cudaMemcpy(sell_ent, e.data(), e.size() * 4, cudaMemcpyHostToDevice));
-        if (!perm.empty()) {
-            V2B_CK(cudaMemcpy(sell_perm, perm.data(), perm.size() * 4, cudaMemcpyHostToDevice));
-            V2B_CK(cudaMemcpy(sell_len, len.data(), len.size(), cudaMemcpyHostToDevice));
-        }
-        V2B_CK(cudaMemcpy(sell_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice));
-    }
-    // Contiguous runs of slices, one per CG warp, of about equal work: a
-    // slice costs its stored entries (32 x its width) plus a fixed share for
-    // its row indices and the write of its results; the long rows, which
-    // warps take round-robin (row k: warp k mod nwarps), count toward their
-    // warp's share.  Warp w's run ends where the cumulative slice work comes
-    // nearest to (w + 1) x the average less the long-row work of warps 0..w
-    // (cumulative targets: the rounding of one warp does not carry into the
-    // next).
-    void split_slices(int64_t nwarps, const v2b::PackedOperator &op) {
-        const double fixed = 32.0 * 3.0;
-        std::vector<double> extra(nwarps, 0.0);
-        int64_t k = 0;
-        double total = 0.0;
-        for (int64_t r = 0; r < op.nrows; r++) {
-            const uint32_t L = op.row_ptr[r + 1] - op.row_ptr[r];
-            if (L <= v2b::kCgLongRow) continue;
-            const double c = 32.0 * (double)((L + 31) / 32) + fixed;
-            extra[k % nwarps] += c;
-            total += c;
-            k++;
-        }
-        std::vector<double> cum(nslices + 1, 0.0);
-        for (int64_t s = 0; s < nslices; s++) cum[s + 1] = cum[s] + (double)(host_off[s + 1] - host_off[s]) + fixed;
-        total += cum[nslices];
-        const double avg = total / (double)nwarps;
-        std::vector<uint32_t> first(nwarps + 1, 0);
-        double ce = 0.0;
-        for (int64_t w = 0; w < nwarps; w++) {
-            ce += extra[w];
-            const double target = (double)(w + 1) * avg - ce;
-            int64_t s = std::lower_bound(cum.begin(), cum.end(), target) - cum.begin();
-            if (s > 0 && s <= nslices && target - cum[s - 1] < cum[s] - target) s--;
-            s = std::min<int64_t>(std::max<int64_t>(s, first[w]), nslices);
-            first[w + 1] = (uint32_t)s;
-        }
-        first[nwarps] = (uint32_t)nslices;
-        if (sell_split) cudaFree(sell_split);
-        sell_split = dalloc<uint32_t>(first.size());
-        V2B_CK(cudaMemcpy(sell_split, first.data(), first.size() * 4, cudaMemcpyHostToDevice));
-    }
-    v2b::SellOp sell() const {
-        v2b::SellOp s;
-        s.ent = sell_ent;
-        s.perm = sell_perm;
-        s.off = sell_off;
-        s.len = sell_len;
-        s.nslices = nslices;
-        s.split = sell_split;
-        return s;
     }
     void release() {
-        for (void *p : {(void *)rp, (void *)ent, (void *)long_rows, (void *)sell_ent, (void *)sell_perm,
-                        (void *)sell_off, (void *)sell_len, (void *)sell_split})
-            cudaFree(p);
-        sell_split = nullptr;
-        rp = ent = sell_ent = sell_perm = sell_off = nullptr;
-        sell_len = nullptr;
-        long_rows = nullptr;
+        for (void *p : {(void *)rp, (void *)ent}) cudaFree(p);
+        rp = ent = nullptr;
+    }
+};
+
+// the CG kernel's tables and vectors on the device (cg_tables.h)
+struct DeviceCg {
+    std::vector<void *> owned;
+    v2b::CgRows dual{}, prim{};
+    uint32_t *orig = nullptr;
+    double2 *rp = nullptr;
+    double *yp = nullptr, *t = nullptr, *slots = nullptr;
+    unsigned int *count = nullptr;
+    int nvirtual = 0, grid = 0;
+    size_t smem = 0;
+    v2b::CgShape shape{};
+
+    template <class T>
+    T *vec(size_t n) {
+        T *d = dalloc<T>(n);
+        owned.push_back(d);
+        return d;
+    }
+    template <class T>
+    T *put(const std::vector<T> &v) {
+        T *d = vec<T>(v.size());
+        if (!v.empty()) V2B_CK(cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+        return d;
+    }
+    v2b::CgRows rows(const v2b::CgSide &s) {
+        v2b::CgRows q;
+        q.off = put(s.off);
+        q.ent = put(s.ent);
+        q.lrp = put(s.lrp);
+        q.lent = put(s.lent);
+        q.split = put(s.split);
+        q.host = put(s.host);
+        q.len = put(s.len);
+        q.nslices = (uint32_t)s.nslices();
+        q.nlong = (uint32_t)s.nlong();
+        return q;
+    }
+    void build(const v2b::PackedOperator &A, const v2b::PackedOperator &AT, int sms) {
+        // Virtual CTAs of 512 threads: a row per thread, three to an SM at most.
+        // They are spread over one CTA per SM; two of them run as one CTA,
+        // without grid barriers.
+        const int64_t want = (std::max(A.nrows, AT.nrows) + 511) / 512;
+        nvirtual = (int)std::max<int64_t>(1, std::min<int64_t>(want, 3 * (int64_t)sms));
+        int v = nvirtual <= 2 ? nvirtual : (nvirtual + sms - 1) / sms;
+        v2b::CgTables h = v2b::build_cg_tables(A, AT, nvirtual, v);
+        // where the tables go: both passes' in shared memory, in turn in one
+        // region of it, or left in global memory ((20e,20o), 47 us per CG
+        // iteration in one region: 63 streamed)
+        auto words = [&](bool both) {   // of the CTA with most
+            size_t most = 0;
+            for (size_t c = 0; c < h.dual.host.size() / v; c++) {
+                size_t sum = 0;
+                for (int w = 0; w < v * v2b::kCgVirtualWarps; w++) {
+                    size_t n[2] = {0, 0};
+                    int k = 0;
+                    for (const v2b::CgSide *s : {&h.dual, &h.prim}) {
+                        const uint32_t vc = s->host[c * v + w / v2b::kCgVirtualWarps];
+                        if (vc != 0xffffffffu) {
+                            const size_t gw = (size_t)vc * v2b::kCgVirtualWarps + w % v2b::kCgVirtualWarps;
+                            n[k] = v2b::cg_table_words(s->split[gw + 1] - s->split[gw],
+                                                       s->at(s->split[gw + 1]) - s->at(s->split[gw]));
+                        }
+                        k++;
+                    }
+                    sum += both ? n[0] + n[1] : std::max(n[0], n[1]);
+                }
+                most = std::max(most, sum);
+            }
+            return most;
+        };
+        const size_t room = (227 * 1024 - v2b::kCgStaticSmem) / 4;
+        v2b::CgTablesIn in = v2b::kCgBoth;
+        smem = 4 * words(true);
+        if (smem > 4 * room && v == 3) {
+            in = v2b::kCgOneRegion;
+            smem = 4 * words(false);
+        }
+        if (smem > 4 * room) {
+            in = v2b::kCgStreamed;
+            smem = 0;
+            if (v != 1) h = v2b::build_cg_tables(A, AT, nvirtual, v = 1);
+        }
+        grid = (nvirtual + v - 1) / v;
+        shape = v2b::cg_shape(v, in);
+        dual = rows(h.dual);
+        prim = rows(h.prim);
+        orig = put(h.dual.orig);
+        rp = vec<double2>(h.dual.rows());
+        yp = vec<double>(h.dual.rows());
+        t = vec<double>(h.prim.rows());
+        slots = vec<double>(2 * (size_t)nvirtual);
+        count = vec<unsigned int>(1);
+        V2B_CK(v2b::raise_dynamic_smem(shape.kernel, (int)smem));
+    }
+    void release() {
+        for (void *q : owned) cudaFree(q);
+        owned.clear();
     }
 };
 
@@ -1269,20 +1251,18 @@ void v2b::set_last_error(const std::string &msg) { g_last_error = msg; }
 struct v2b_problem {
     v2b::Problem prob;
     DeviceOp A, AT;
+    DeviceCg cg;
     ProjectPlan plan;
     cudaStream_t stream = nullptr;
     double *x = nullptr, *b = nullptr, *c = nullptr, *y = nullptr, *z = nullptr;
     double *Ax = nullptr, *Acz = nullptr, *ATy = nullptr, *U = nullptr;
-    double *r = nullptr, *p0 = nullptr, *p1 = nullptr, *t = nullptr;
     double *y1 = nullptr, *y2 = nullptr;   // the last two dual solutions, for the CG start
-    double *partials = nullptr, *cg_out = nullptr, *stats = nullptr, *stats_partials = nullptr;
+    double *cg_out = nullptr, *stats = nullptr, *stats_partials = nullptr;
     unsigned int *stats_counter = nullptr;
-    v2b::GridBarrier *bar = nullptr;
     int *ibas_aa_dev = nullptr;   // n x n aa geminal numbers, for the density packing
     double *pack_layout = nullptr;   // DOCI: x in the v2RDM layout, for the density packing
     int *status = nullptr;   // [0] fatal device status, [1] projection sweeps exhausted
     double *h_readback = nullptr;   // pinned: stats[4], cg_out[2], status[2]
-    int cg_grid = 0;
     double mu = 0.1;
     long launches = 0;
     long cur_oiter = 0;
@@ -1331,14 +1311,14 @@ struct v2b_problem {
         if (!on_device) return;
         A.release();
         AT.release();
+        cg.release();
         plan.release();
-        for (double *p : {x, b, c, y, z, Ax, Acz, ATy, U, r, p0, p1, t, y1, y2, partials, cg_out, stats,
+        for (double *p : {x, b, c, y, z, Ax, Acz, ATy, U, y1, y2, cg_out, stats,
                           stats_partials})
             cudaFree(p);
         if (cg_phase) cudaFree(cg_phase);
         if (pack_layout) cudaFree(pack_layout);
         cudaFree(stats_counter);
-        cudaFree(bar);
         cudaFree(ibas_aa_dev);
         cudaFree(status);
         if (nonfinite) cudaFree(nonfinite);
@@ -1373,27 +1353,15 @@ struct v2b_problem {
         AT.upload(hostAT);
         const int64_t np = prob.n_primal, nd = prob.n_dual;
         x = dalloc<double>(np); c = dalloc<double>(np); z = dalloc<double>(np);
-        ATy = dalloc<double>(np); U = dalloc<double>(np); t = dalloc<double>(np);
+        ATy = dalloc<double>(np); U = dalloc<double>(np);
         b = dalloc<double>(nd); y = dalloc<double>(nd); Ax = dalloc<double>(nd);
-        Acz = dalloc<double>(nd); r = dalloc<double>(nd); p0 = dalloc<double>(nd);
-        p1 = dalloc<double>(nd);
+        Acz = dalloc<double>(nd);
         y1 = dalloc<double>(nd); y2 = dalloc<double>(nd);
-        int per_sm = 0;
-        V2B_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v2b::cg_kernel,
-                                                             v2b::kCgThreads, 0));
-        if (per_sm < 1) throw Failure(V2B_INTERNAL, "cg_kernel cannot be resident");
-        // small problems: fewer CTAs make the grid barrier cheaper
-        const int64_t rows = std::max(prob.n_primal, prob.n_dual);
-        const int64_t want = (rows + (int64_t)v2b::kCgThreads - 1) / (int64_t)v2b::kCgThreads;
-        cg_grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count() * per_sm));
-        A.split_slices((int64_t)cg_grid * (v2b::kCgThreads / 32), hostA);
-        AT.split_slices((int64_t)cg_grid * (v2b::kCgThreads / 32), hostAT);
-        partials = dalloc<double>(2 * (size_t)cg_grid);
+        cg.build(hostA, hostAT, sm_count());
         stats_partials = dalloc<double>(4 * v2b::kStatsBlocks);
         cg_out = dalloc<double>(2);
         stats = dalloc<double>(4);
         stats_counter = dalloc<unsigned int>(1);
-        bar = dalloc<v2b::GridBarrier>(1);
         status = dalloc<int>(2);
         V2B_CK(cudaMemset(stats_counter, 0, 4));
         V2B_CK(cudaMemset(status, 0, 8));
@@ -1424,23 +1392,21 @@ struct v2b_problem {
     }
 
     void launch_cg(double tol, int maxit) {
-        V2B_CK(cudaMemsetAsync(bar, 0, sizeof(v2b::GridBarrier), stream));
+        V2B_CK(cudaMemsetAsync(cg.count, 0, sizeof(unsigned int), stream));
         v2b::CgParams P;
-        P.a_rp = A.rp; P.a_ent = A.ent; P.t_rp = AT.rp; P.t_ent = AT.ent;
-        P.long_a = A.long_rows; P.long_t = AT.long_rows;
-        P.n_long_a = A.n_long; P.n_long_t = AT.n_long;
-        P.sa = A.sell(); P.st = AT.sell();
+        P.dual = cg.dual; P.prim = cg.prim; P.orig = cg.orig;
         P.palA = A.pal; P.palT = AT.pal;
-        P.np = prob.n_primal; P.nd = prob.n_dual;
         P.Ax = Ax; P.Acz = Acz; P.b = b; P.mu = mu;
-        P.y = y; P.r = r; P.p0 = p0; P.p1 = p1; P.t = t;
-        P.partials = partials; P.bar = bar; P.status = status;
+        P.y = y; P.rp = cg.rp; P.yp = cg.yp; P.t = cg.t;
+        P.slots = cg.slots; P.count = cg.count; P.status = status;
         P.spin_limit = wait_limit;
-        P.tol = tol; P.maxit = maxit; P.out = cg_out;
+        P.tol = tol; P.maxit = maxit;
+        P.nvirtual = cg.nvirtual;
+        P.out = cg_out;
         P.phase_ns = (profiling && phases) ? cg_phase : nullptr;
         void *args[] = {&P};
-        V2B_CK(cudaLaunchCooperativeKernel((const void *)v2b::cg_kernel, dim3(cg_grid),
-                                           dim3(v2b::kCgThreads), args, 0, stream));
+        V2B_CK(cudaLaunchCooperativeKernel(cg.shape.kernel, dim3(cg.grid), dim3(cg.shape.threads), args, cg.smem,
+                                           stream));
         launches++;
     }
 

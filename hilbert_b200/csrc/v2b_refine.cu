@@ -35,6 +35,8 @@
 #include "v2b_kernels.cuh"
 #include "v2b_refine.cuh"
 
+#include <algorithm>
+
 namespace v2b {
 
 __device__ __forceinline__ double gamma_pq(double li, double lj) {
@@ -181,39 +183,96 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------- clusters
-// Cyclic Jacobi on one cluster per CTA (k <= kRefineSmallCluster), A and the
-// eigenvector rows Q in shared memory.  The round-robin pairs of every step
-// are tabulated once; a step computes the rotations of its m = kp/2 disjoint
-// pairs (sym.schur2), then applies all of them at once, each thread updating
-// whole 2 x 2 blocks (rows of pair P, columns of pair Q) two-sidedly and the
-// rows p, q of Q: two barriers per step.
-__global__ void __launch_bounds__(256)
+// Cyclic Jacobi on one cluster (k <= kRefineSmallCluster), A and the
+// eigenvector rows Q in shared memory.  A step takes the m = kp / 2 disjoint
+// round-robin pairs (sym.schur2 rotations), each 2 x 2 block (rows of pair P,
+// columns of pair Q2) two-sidedly, and the rows p, q of Q.
+//
+// A step is a chain: the rotations' divisions and roots (600 cycles alone),
+// then the update, which is bound by shared memory (every element of A and Q
+// is read and written).  So the chain runs beside the update: a warp of its
+// own forms the three elements that each next pair needs from the blocks as
+// they stand before the update, then the next rotations, while the others
+// write A and update Q; they wait only until it has read.  And the columns of
+// Q are cut over `slices` CTAs, each of which repeats the whole of A (the same
+// bits): no exchange, and Q's traffic, half of a step's, is divided.  A
+// 64-row job, two sweeps: 216 us with the rotations and the updates in turn
+// and one CTA a job, 137 us so.
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+struct RotBlock {
+    double n11, n12, n21, n22;
+};
+// the 2 x 2 block b of pairs (P, Q2) after both rotations; same: P == Q2, the
+// pair's own coupling is annihilated
+__device__ __forceinline__ RotBlock rotate_block(double b11, double b12, double b21, double b22, double2 cp,
+                                                 double2 cq, bool same) {
+    const double m11 = b11 * cq.x - b12 * cq.y, m12 = b11 * cq.y + b12 * cq.x;
+    const double m21 = b21 * cq.x - b22 * cq.y, m22 = b21 * cq.y + b22 * cq.x;
+    RotBlock r;
+    r.n11 = cp.x * m11 - cp.y * m21;
+    r.n12 = cp.x * m12 - cp.y * m22;
+    r.n21 = cp.y * m11 + cp.x * m21;
+    r.n22 = cp.y * m12 + cp.x * m22;
+    if (same) r.n12 = r.n21 = 0.0;
+    return r;
+}
+// rr_pair without divisions, and its inverse: the pair that holds index j
+__device__ __forceinline__ void rr_pair_fast(int s, int k, int m1, int &p, int &q) {
+    int a = s + k, b = s - k;
+    a = a >= m1 ? a - m1 : a;
+    b = b < 0 ? b + m1 : b;
+    a = k == 0 ? m1 : a;
+    p = min(a, b);
+    q = max(a, b);
+}
+// what the rotating warp needs of step st for pair `lane` of the next step
+// (p, q): each index's partner and pair in step st
+__device__ __forceinline__ uint2 next_pair_entry(int st, int nx, int lane, int m1) {
+    auto pair_of = [&](int j) {
+        if (j == m1 || j == st) return 0;
+        const int d = j > st ? j - st : j - st + m1;
+        return min(d, m1 - d);
+    };
+    int p, q, a, b, c, d;
+    rr_pair_fast(nx, lane, m1, p, q);
+    const int Pp = pair_of(p), Pq = pair_of(q);
+    rr_pair_fast(st, Pp, m1, a, b);
+    rr_pair_fast(st, Pq, m1, c, d);
+    return make_uint2((unsigned)(p | (a + b - p) << 8 | Pp << 16), (unsigned)(q | (c + d - q) << 8 | Pq << 16));
+}
+
+// NT threads update, a warp per pair row P and a lane per pair column; one more
+// warp rotates.  NT = 128: at most 32 rows (16 pairs).
+template <int NT>
+__global__ void __launch_bounds__(NT + 32)
     cluster_eig_kernel(const double *__restrict__ T, const int64_t *__restrict__ boff,
                        const int *__restrict__ bdim, const ClusterJob *__restrict__ jobs,
                        const int *__restrict__ mem, double *__restrict__ Qt,
-                       double *__restrict__ lam, const int *__restrict__ only, int max_sweeps) {
-    const ClusterJob jb = jobs[blockIdx.x];
+                       double *__restrict__ lam, const int *__restrict__ only, int max_sweeps, int slices) {
+    const ClusterJob jb = jobs[blockIdx.x / slices];
     if (only && !only[jb.blk]) return;   // uniform over the CTA
+    constexpr int KM = kRefineSmallCluster, WARPS = NT / 32, PASSES = 2 * (NT > 128 ? 16 : 8) / WARPS;
     const int k = jb.k, n = bdim[jb.blk];
     const int kp = k + (k & 1), ld = kp + 1, m = kp / 2, nst = kp - 1;
+    // this CTA's columns of Q
+    const int cw = (kp + slices - 1) / slices, c0 = (int)(blockIdx.x % slices) * cw, c1 = min(kp, c0 + cw);
+    if (c0 >= c1 && c0 > 0) return;   // uniform over the CTA
     const int *C = mem + jb.moff;
     const double *Tb = T + boff[jb.blk];
     extern __shared__ double sm[];
     double *A = sm;              // kp x ld
-    double *Q = A + kp * ld;     // kp x ld, rows = eigenvectors
-    constexpr int KM = kRefineSmallCluster;
-    __shared__ unsigned char pr[KM - 1][KM / 2], qr[KM - 1][KM / 2];
-    __shared__ double2 cs[KM / 2];
+    double *Q = A + kp * ld;     // kp x cw, rows = eigenvectors
+    uint2 *next = (uint2 *)(Q + kp * cw);   // nst x m
+    __shared__ double2 cs[3][KM / 2];   // the step before, this one, the next
     __shared__ double red[32];
     __shared__ double s_thr;
-    __shared__ int s_nrot;
+    __shared__ int s_any[2];
     const int tid = threadIdx.x;
-    for (int e = tid; e < nst * m; e += blockDim.x) {
-        int p, q;
-        rr_pair(e / m, e % m, kp, p, q);
-        pr[e / m][e % m] = (unsigned char)p;
-        qr[e / m][e % m] = (unsigned char)q;
-    }
     double fro = 0.0;
     for (int e = tid; e < kp * kp; e += blockDim.x) {
         const int i = e / kp, j = e % kp;
@@ -223,8 +282,12 @@ __global__ void __launch_bounds__(256)
             v = 0.5 * (Tb[a * n + b] + Tb[b * n + a]);
         }
         A[i * ld + j] = v;
-        Q[i * ld + j] = (i == j) ? 1.0 : 0.0;
+        if (j >= c0 && j < c1) Q[i * cw + j - c0] = (i == j) ? 1.0 : 0.0;
         fro += v * v;
+    }
+    for (int e = tid; e < nst * m; e += blockDim.x) {
+        const int st = e / m;
+        next[e] = next_pair_entry(st, st + 1 < nst ? st + 1 : 0, e % m, nst);
     }
     fro = block_sum(fro, red);
     // rotate down to 1e-14 of the cluster's norm: below the acceptance test's
@@ -233,71 +296,210 @@ __global__ void __launch_bounds__(256)
     if (tid == 0) s_thr = 1e-14 * sqrt(fro) + 1e-300;
     __syncthreads();
     const double thr = s_thr;
-    const int P = tid >> 3, sub = tid & 7;   // 32 pair rows x 8 lanes
-    for (int sweep = 0; sweep < max_sweeps; sweep++) {
-        if (tid == 0) s_nrot = 0;
-        __syncthreads();
-        for (int st = 0; st < nst; st++) {
-            if (tid < m) {
-                const int p = pr[st][tid], q = qr[st][tid];
-                double c = 1.0, s = 0.0;
-                if (q < k) {
-                    const double apq = A[p * ld + q];
-                    if (fabs(apq) > thr) {
-                        const double app = A[p * ld + p], aqq = A[q * ld + q];
-                        const double tau = (aqq - app) / (2.0 * apq);
-                        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + hypot(1.0, tau));
-                        c = 1.0 / sqrt(1.0 + t * t);
-                        s = t * c;
-                        atomicAdd(&s_nrot, 1);
-                    }
-                }
-                cs[tid] = make_double2(c, s);
-            }
-            __syncthreads();
-            if (P < m) {
-                const double2 cp = cs[P];
-                const int pP = pr[st][P], qP = qr[st][P];
-                // A <- G A G^T on the 2 x 2 blocks (P, Q2)
-                for (int Q2 = sub; Q2 < m; Q2 += 8) {
-                    const double2 cq = cs[Q2];
-                    if (cp.y == 0.0 && cq.y == 0.0) continue;
-                    const int pQ = pr[st][Q2], qQ = qr[st][Q2];
-                    const double b11 = A[pP * ld + pQ], b12 = A[pP * ld + qQ];
-                    const double b21 = A[qP * ld + pQ], b22 = A[qP * ld + qQ];
-                    const double m11 = b11 * cq.x - b12 * cq.y, m12 = b11 * cq.y + b12 * cq.x;
-                    const double m21 = b21 * cq.x - b22 * cq.y, m22 = b21 * cq.y + b22 * cq.x;
-                    double n11 = cp.x * m11 - cp.y * m21, n12 = cp.x * m12 - cp.y * m22;
-                    double n21 = cp.y * m11 + cp.x * m21, n22 = cp.y * m12 + cp.x * m22;
-                    if (Q2 == P) n12 = n21 = 0.0;   // the pair's own coupling, annihilated
-                    A[pP * ld + pQ] = n11;
-                    A[pP * ld + qQ] = n12;
-                    A[qP * ld + pQ] = n21;
-                    A[qP * ld + qQ] = n22;
-                }
-                // Q <- G Q on rows p, q
-                if (cp.y != 0.0)
-                    for (int jc = sub; jc < kp; jc += 8) {
-                        const double qp = Q[pP * ld + jc], qq = Q[qP * ld + jc];
-                        Q[pP * ld + jc] = cp.x * qp - cp.y * qq;
-                        Q[qP * ld + jc] = cp.y * qp + cp.x * qq;
-                    }
-            }
-            __syncthreads();
+    const int m1 = nst;
+    // the rotation of the pair with elements app, aqq, apq (q < k: not padding)
+    auto rotation = [&](int q, double app, double aqq, double apq) {
+        double c = 1.0, s = 0.0;
+        if (q < k && fabs(apq) > thr) {
+            const double tau = (aqq - app) / (2.0 * apq);
+            // a correctly rounded reciprocal is 1.0 / x, in half the time
+            const double r = __drcp_rn(fabs(tau) + hypot(1.0, tau)), t = tau >= 0.0 ? r : -r;
+            c = 1.0 / sqrt(1.0 + t * t);
+            s = t * c;
         }
-        const int nrot = s_nrot;   // read by all before thread 0 resets it
+        return make_double2(c, s);
+    };
+    if (tid >= NT) {   // the rotating warp; its lanes keep this step's rotations
+        const int lane = tid - NT;
+        double2 mine = make_double2(1.0, 0.0);
+        bool any = false;   // a pair was rotated in this sweep
+        if (lane < m) {
+            int p, q;
+            rr_pair_fast(0, lane, m1, p, q);
+            mine = rotation(q, A[p * ld + p], A[q * ld + q], A[p * ld + q]);
+            cs[0][lane] = mine;
+            any = mine.y != 0.0;
+        }
         __syncthreads();
-        if (nrot == 0) break;
+        int cur = 0;
+        uint2 e = lane < m ? next[lane] : make_uint2(0u, 0u);
+        for (int sweep = 0; sweep < max_sweeps; sweep++) {
+            for (int st = 0; st < nst; st++) {
+                const int p = e.x & 255, p2 = (e.x >> 8) & 255, Pp = e.x >> 16;
+                const int q = e.y & 255, q2 = (e.y >> 8) & 255, Pq = e.y >> 16;
+                const double2 cp = make_double2(__shfl_sync(0xffffffffu, mine.x, Pp), __shfl_sync(0xffffffffu, mine.y, Pp));
+                const double2 cq = make_double2(__shfl_sync(0xffffffffu, mine.x, Pq), __shfl_sync(0xffffffffu, mine.y, Pq));
+                const int pp = min(p, p2), pq = max(p, p2), qp = min(q, q2), qq = max(q, q2);
+                // rows and columns (pp, pq) x (pp, pq), (qp, qq) x (qp, qq) and
+                // (pp, pq) x (qp, qq) of A as they stand
+                const double a11 = A[pp * ld + pp], a12 = A[pp * ld + pq], a21 = A[pq * ld + pp], a22 = A[pq * ld + pq];
+                const double b11 = A[qp * ld + qp], b12 = A[qp * ld + qq], b21 = A[qq * ld + qp], b22 = A[qq * ld + qq];
+                const double x11 = A[pp * ld + qp], x12 = A[pp * ld + qq], x21 = A[pq * ld + qp], x22 = A[pq * ld + qq];
+                const RotBlock ra = rotate_block(a11, a12, a21, a22, cp, cp, true);
+                const RotBlock rb = rotate_block(b11, b12, b21, b22, cq, cq, true);
+                const RotBlock rx = rotate_block(x11, x12, x21, x22, cp, cq, Pp == Pq && cp.y != 0.0);
+                const double app = p == pp ? ra.n11 : ra.n22, aqq = q == qp ? rb.n11 : rb.n22;
+                const double lo = q == qp ? rx.n11 : rx.n12, hi = q == qp ? rx.n21 : rx.n22;
+                const double apq = p == pp ? lo : hi;
+                bar_arrive(1, NT + 32);   // this step's A has been read
+                // the next sweep's rotations begin in this sweep's last step
+                if (st + 1 == nst) {
+                    const int rotated = __any_sync(0xffffffffu, any);
+                    if (lane == 0) s_any[sweep & 1] = rotated;
+                    any = false;
+                }
+                if (lane < m) {
+                    mine = rotation(q, app, aqq, apq);
+                    cs[cur == 2 ? 0 : cur + 1][lane] = mine;
+                    any = any || mine.y != 0.0;
+                    e = next[(st + 1 < nst ? st + 1 : 0) * m + lane];
+                }
+                __syncwarp();
+                cur = cur == 2 ? 0 : cur + 1;
+                __syncthreads();
+            }
+            if (!s_any[sweep & 1]) break;
+        }
+    } else {
+        __syncthreads();
+        const int warp = tid >> 5, lane = tid & 31;
+        const bool col = lane < m;   // this lane has a pair column
+        // Q <- G Q of step st, rotations cs[c], this CTA's columns: the warp's
+        // pair rows side by side over its lanes
+        auto update_Q = [&](int st, int c) {
+            for (int f = lane; f < PASSES * cw; f += 32) {
+                const int i = f / cw, jc = f - i * cw, P = warp + i * WARPS;
+                if (P >= m || jc >= c1 - c0) continue;
+                const double2 g = cs[c][P];
+                if (g.y == 0.0) continue;
+                int p, q;
+                rr_pair_fast(st, P, m1, p, q);
+                const double qp = Q[p * cw + jc], qq = Q[q * cw + jc];
+                Q[p * cw + jc] = g.x * qp - g.y * qq;
+                Q[q * cw + jc] = g.y * qp + g.x * qq;
+            }
+        };
+        int cur = 0, last = -1;   // last: the step whose rotations Q still lacks
+        for (int sweep = 0; sweep < max_sweeps; sweep++) {
+            for (int st = 0; st < nst; st++) {
+                // Q first: the rotating warp's reads of A go ahead of these warps'
+                if (last >= 0) update_Q(last, cur == 0 ? 2 : cur - 1);
+                // A <- G A G^T on the 2 x 2 blocks (P, lane), held until all are
+                // read.  Without a rotation a block comes out as it went in.
+                RotBlock r[PASSES];
+                int pP[PASSES], qP[PASSES], pQ, qQ;
+                double2 cp[PASSES];
+                const double2 cq = cs[cur][col ? lane : 0];
+                rr_pair_fast(st, col ? lane : 0, m1, pQ, qQ);
+#pragma unroll
+                for (int i = 0; i < PASSES; i++) {
+                    const int P = min(warp + i * WARPS, m - 1);
+                    cp[i] = cs[cur][P];
+                    rr_pair_fast(st, P, m1, pP[i], qP[i]);
+                }
+                double a[PASSES][4];
+#pragma unroll
+                for (int i = 0; i < PASSES; i++) {
+                    a[i][0] = A[pP[i] * ld + pQ];
+                    a[i][1] = A[pP[i] * ld + qQ];
+                    a[i][2] = A[qP[i] * ld + pQ];
+                    a[i][3] = A[qP[i] * ld + qQ];
+                }
+#pragma unroll
+                for (int i = 0; i < PASSES; i++)
+                    r[i] = rotate_block(a[i][0], a[i][1], a[i][2], a[i][3], cp[i], cq,
+                                        lane == warp + i * WARPS && cq.y != 0.0);
+                bar_sync(1, NT + 32);
+#pragma unroll
+                for (int i = 0; i < PASSES; i++)
+                    if (col && warp + i * WARPS < m) {
+                        A[pP[i] * ld + pQ] = r[i].n11;
+                        A[pP[i] * ld + qQ] = r[i].n12;
+                        A[qP[i] * ld + pQ] = r[i].n21;
+                        A[qP[i] * ld + qQ] = r[i].n22;
+                    }
+                last = st;
+                cur = cur == 2 ? 0 : cur + 1;
+                __syncthreads();
+            }
+            if (!s_any[sweep & 1]) break;
+        }
+        if (last >= 0) update_Q(last, cur == 0 ? 2 : cur - 1);
     }
+    __syncthreads();
     double *Qo = Qt + jb.qoff;
-    for (int e = tid; e < k * k; e += blockDim.x) Qo[e] = Q[(e / k) * ld + e % k];
-    for (int i = tid; i < k; i += blockDim.x) lam[jb.moff + i] = A[i * ld + i];
+    for (int e = tid; e < k * cw; e += blockDim.x) {
+        const int i = e / cw, j = c0 + e % cw;
+        if (j < min(k, c1)) Qo[i * k + j] = Q[i * cw + e % cw];
+    }
+    if (c0 == 0)
+        for (int i = tid; i < k; i += blockDim.x) lam[jb.moff + i] = A[i * ld + i];
+}
+
+// A, Q and the table of next pairs (one 8-byte entry per pair and step)
+static size_t cluster_eig_smem(int kp, int cw) {
+    return sizeof(double) * ((size_t)kp * (kp + 1) + (size_t)kp * cw + (size_t)(kp - 1) * (kp / 2));
+}
+
+cudaError_t launch_cluster_eig(int njobs, int kmax, int sms, cudaStream_t s, const double *T, const int64_t *boff,
+                               const int *bdim, const ClusterJob *jobs, const int *mem, double *Qt, double *lam,
+                               const int *only, int max_sweeps) {
+    if (njobs <= 0) return cudaSuccess;
+    const int kp = kmax + (kmax & 1);
+    // columns of Q over as many CTAs as the SMs hold at once, at least 16 each
+    const int slices = std::max(1, std::min({4, kp / 16, sms / njobs}));
+    const size_t smem = cluster_eig_smem(kp, (kp + slices - 1) / slices);
+    if (kp > 32)
+        cluster_eig_kernel<512><<<njobs * slices, 512 + 32, smem, s>>>(T, boff, bdim, jobs, mem, Qt, lam, only,
+                                                                      max_sweeps, slices);
+    else
+        cluster_eig_kernel<128><<<njobs * slices, 128 + 32, smem, s>>>(T, boff, bdim, jobs, mem, Qt, lam, only,
+                                                                      max_sweeps, slices);
+    return cudaGetLastError();
+}
+
+cudaError_t prepare_cluster_eig() {
+    const int kc = kRefineSmallCluster;
+    const int smem = (int)cluster_eig_smem(kc, kc);
+    cudaError_t e = raise_dynamic_smem((const void *)cluster_eig_kernel<512>, smem);
+    return e == cudaSuccess ? raise_dynamic_smem((const void *)cluster_eig_kernel<128>, smem) : e;
 }
 
 // One block-Jacobi step applied in place.  The step's jobs partition each
 // block's rows, so T splits into job tiles T[C_I, C_J] that only their own
 // CTA reads and writes:  tile kind 0 (I, J):  T[C_I, C_J] <- Qt_I T[C_I, C_J] Qt_J^T;
 // kind 1 (I, t):  Vt[C_I, 64 t .. 64 t + 64) <- Qt_I Vt[C_I, ...].
+//
+// 64 x 64 x 64 products on FP64 tensor cores (m8n8k4; its four products
+// accumulate in ascending k with one rounding each, bit for bit an FMA chain),
+// eight warps of 32 x 16 each: 8 fragment loads feed 8 MMAs, where FMAs from
+// shared memory were bound by their operand loads (45 us a launch at 200 rows
+// then, 25 now with cold caches; 4 us of it are the MMAs of one tile).
+constexpr int kBjLd = kRefineSmallCluster + 4;   // rows 4 doubles apart mod 16: fragments free of conflicts
+
+// c += op(X) Y over K = 64 (zero-padded): rows wm.., columns wn..; X row-major
+// 64 x 64; Y row-major (k x n), or with YT its transpose (n x k)
+template <bool YT>
+__device__ __forceinline__ void bj_mma(const double *X, const double *Y, int wm, int wn, int lane, int kmax,
+                                       double (&c)[4][2][2]) {
+    const int fr = lane >> 2, fk = lane & 3;
+    for (int k = 0; k < kmax; k += 4) {
+        double x[4], y[2];
+#pragma unroll
+        for (int i = 0; i < 4; i++) x[i] = X[(wm + 8 * i + fr) * kBjLd + k + fk];
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            y[j] = YT ? Y[(wn + 8 * j + fr) * kBjLd + k + fk] : Y[(k + fk) * kBjLd + wn + 8 * j + fr];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                             : "+d"(c[i][j][0]), "+d"(c[i][j][1])
+                             : "d"(x[i]), "d"(y[j]));
+    }
+}
+
 __global__ void __launch_bounds__(256)
     bj_apply_kernel(double *__restrict__ T, double *__restrict__ Vt, const int64_t *__restrict__ boff,
                     const int *__restrict__ bdim, const ClusterJob *__restrict__ jobs,
@@ -308,96 +510,66 @@ __global__ void __launch_bounds__(256)
     if (only && !only[jI.blk]) return;   // uniform over the CTA
     const int n = bdim[jI.blk];
     const int64_t off = boff[jI.blk];
-    constexpr int KM = kRefineSmallCluster, LD = KM + 1;
+    constexpr int KM = kRefineSmallCluster, SZ = KM * kBjLd;
     extern __shared__ double sm[];
-    double *sQ = sm;              // KM x LD: Qt_I
-    double *sX = sQ + KM * LD;    // KM x LD: the tile, then Qt_I x tile
-    double *sR = sX + KM * LD;    // KM x LD: Qt_J (kind 0)
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    double *sQ = sm;              // Qt_I, zero past its kI rows and columns
+    double *sX = sm + SZ;         // the tile, then Qt_I x tile
+    double *sR = sm + 2 * SZ;     // Qt_J (kind 0)
+    __shared__ int rI[KM], rJ[KM];   // global rows; columns of kind 1
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
     const int kI = jI.k;
-    const int *CI = mem + jI.moff;
-    for (int e = tid; e < kI * kI; e += blockDim.x) sQ[(e / kI) * LD + e % kI] = Qt[jI.qoff + e];
-    if (tl.z == 0) {
-        const ClusterJob jJ = jobs[tl.y];
-        const int kJ = jJ.k;
-        const int *CJ = mem + jJ.moff;
-        for (int e = tid; e < kJ * kJ; e += blockDim.x) sR[(e / kJ) * LD + e % kJ] = Qt[jJ.qoff + e];
-        for (int e = tid; e < kI * kJ; e += blockDim.x) {
-            const int i = e / kJ, j = e % kJ;
-            sX[i * LD + j] = T[off + (int64_t)CI[i] * n + CJ[j]];
-        }
-        __syncthreads();
-        // Y = Qt_I X (rows 4 ty .., cols 4 tx ..)
-        double y[4][4] = {};
-        for (int l = 0; l < kI; l++) {
-            double a[4], b[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) a[r] = (4 * ty + r < kI) ? sQ[(4 * ty + r) * LD + l] : 0.0;
-#pragma unroll
-            for (int c = 0; c < 4; c++) b[c] = (4 * tx + c < kJ) ? sX[l * LD + 4 * tx + c] : 0.0;
-#pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) y[r][c] = fma(a[r], b[c], y[r][c]);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) sX[(4 * ty + r) * LD + 4 * tx + c] = y[r][c];
-        __syncthreads();
-        // Z = Y Qt_J^T
-        double z[4][4] = {};
-        for (int l = 0; l < kJ; l++) {
-            double a[4], b[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) a[r] = sX[(4 * ty + r) * LD + l];
-#pragma unroll
-            for (int c = 0; c < 4; c++) b[c] = (4 * tx + c < kJ) ? sR[(4 * tx + c) * LD + l] : 0.0;
-#pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) z[r][c] = fma(a[r], b[c], z[r][c]);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int i = 4 * ty + r;
-            if (i >= kI) continue;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int j = 4 * tx + c;
-                if (j < kJ) T[off + (int64_t)CI[i] * n + CJ[j]] = z[r][c];
-            }
-        }
+    const bool two = tl.z == 0;
+    int kJ = 64;
+    if (tid < KM) rI[tid] = tid < kI ? mem[jI.moff + tid] : 0;
+    ClusterJob jJ = jI;
+    if (two) {
+        jJ = jobs[tl.y];
+        kJ = jJ.k;
+        if (tid < KM) rJ[tid] = tid < kJ ? mem[jJ.moff + tid] : 0;
     } else {
         const int c0 = tl.y * 64;
-        for (int e = tid; e < kI * 64; e += blockDim.x) {
-            const int i = e >> 6, c = c0 + (e & 63);
-            sX[i * LD + (e & 63)] = (c < n) ? Vt[off + (int64_t)CI[i] * n + c] : 0.0;
-        }
+        kJ = min(64, n - c0);
+        if (tid < KM) rJ[tid] = c0 + min(tid, kJ - 1);
+    }
+    __syncthreads();
+    double *G = (two ? T : Vt) + off;
+#pragma unroll 8
+    for (int e = tid; e < KM * KM; e += 256) {
+        const int i = e >> 6, j = e & 63;
+        sQ[i * kBjLd + j] = i < kI && j < kI ? Qt[jI.qoff + i * kI + j] : 0.0;
+        sX[i * kBjLd + j] = i < kI && j < kJ ? G[(int64_t)rI[i] * n + rJ[j]] : 0.0;
+        if (two) sR[i * kBjLd + j] = i < kJ && j < kJ ? Qt[jJ.qoff + i * kJ + j] : 0.0;
+    }
+    __syncthreads();
+    const int fr = lane >> 2, fk = lane & 3;
+    double c[4][2][2] = {};
+    bj_mma<false>(sQ, sX, wm, wn, lane, (kI + 3) & ~3, c);   // Y = Qt_I X
+    if (two) {
         __syncthreads();
-        double y[4][4] = {};
-        for (int l = 0; l < kI; l++) {
-            double a[4], b[4];
 #pragma unroll
-            for (int r = 0; r < 4; r++) a[r] = (4 * ty + r < kI) ? sQ[(4 * ty + r) * LD + l] : 0.0;
+        for (int i = 0; i < 4; i++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) b[c] = sX[l * LD + 4 * tx + c];
+            for (int j = 0; j < 2; j++)
 #pragma unroll
-            for (int r = 0; r < 4; r++)
+                for (int h = 0; h < 2; h++) {
+                    sX[(wm + 8 * i + fr) * kBjLd + wn + 8 * j + 2 * fk + h] = c[i][j][h];
+                    c[i][j][h] = 0.0;
+                }
+        __syncthreads();
+        bj_mma<true>(sX, sR, wm, wn, lane, (kJ + 3) & ~3, c);   // Z = Y Qt_J^T
+    }
 #pragma unroll
-                for (int c = 0; c < 4; c++) y[r][c] = fma(a[r], b[c], y[r][c]);
-        }
+    for (int i = 0; i < 4; i++) {
+        const int r = wm + 8 * i + fr;
+        if (r >= kI) continue;
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int i = 4 * ty + r;
-            if (i >= kI) continue;
+        for (int j = 0; j < 2; j++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int cc = c0 + 4 * tx + c;
-                if (cc < n) Vt[off + (int64_t)CI[i] * n + cc] = y[r][c];
+            for (int h = 0; h < 2; h++) {
+                const int q = wn + 8 * j + 2 * fk + h;
+                if (q < kJ) G[(int64_t)rI[r] * n + rJ[q]] = c[i][j][h];
             }
-        }
     }
 }
 

@@ -57,12 +57,12 @@ __global__ void write_p_kernel(const double *__restrict__ T, double *__restrict_
 
 // cyclic Jacobi on each cluster's T[C, C] (at most max_sweeps sweeps; enough
 // sweeps diagonalise it exactly): rows of Qt (k x k) are the eigenvectors,
-// lam the diagonal left
-__global__ void cluster_eig_kernel(const double *__restrict__ T, const int64_t *__restrict__ boff,
-                                   const int *__restrict__ bdim, const ClusterJob *__restrict__ jobs,
-                                   const int *__restrict__ mem, double *__restrict__ Qt,
-                                   double *__restrict__ lam, const int *__restrict__ only,
-                                   int max_sweeps);
+// lam the diagonal left.  kmax: the largest job's rows (<= kRefineSmallCluster).
+cudaError_t launch_cluster_eig(int njobs, int kmax, int sms, cudaStream_t s, const double *T, const int64_t *boff,
+                               const int *bdim, const ClusterJob *jobs, const int *mem, double *Qt, double *lam,
+                               const int *only, int max_sweeps);
+// the kernels' shared-memory limits, once per device before the first launch
+cudaError_t prepare_cluster_eig();
 
 // gathered GEMM tiles of the cluster transform; ctiles = (job, tile row, tile col).
 // With `only` non-null, jobs of blocks b with only[b] == 0 are skipped.
@@ -88,7 +88,8 @@ __global__ void cluster_commit_kernel(double *__restrict__ T, const double *__re
                                       const int *__restrict__ only);
 // one block-Jacobi step in place: tiles (I, J, 0) T[C_I, C_J] <- Qt_I T Qt_J^T,
 // (I, t, 1) Vt[C_I, 64 t ..] <- Qt_I Vt[C_I, ..]; dynamic shared memory
-// 3 x 64 x 65 doubles
+// kBjApplySmem
+constexpr int kBjApplySmem = 3 * kRefineSmallCluster * (kRefineSmallCluster + 4) * (int)sizeof(double);
 __global__ void bj_apply_kernel(double *__restrict__ T, double *__restrict__ Vt,
                                 const int64_t *__restrict__ boff, const int *__restrict__ bdim,
                                 const ClusterJob *__restrict__ jobs, const int *__restrict__ mem,

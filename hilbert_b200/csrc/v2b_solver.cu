@@ -98,6 +98,13 @@ void ensure_device() {
         throw Failure(V2B_NO_DEVICE, "no CUDA device available");
 }
 
+int sm_count() {
+    int dev = 0, n = 0;
+    V2B_CK(cudaGetDevice(&dev));
+    V2B_CK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    return n;
+}
+
 struct DeviceOp {
     uint32_t *rp = nullptr, *ent = nullptr;
     int64_t nrows = 0;
@@ -240,7 +247,7 @@ struct ProjectPlan {
     std::vector<int> dims;
     std::vector<int64_t> h_off;
     std::vector<int64_t> h_roff_small, h_roff_big;   // per block, -1 if not of that kind
-    int nblk = 0, nsmall = 0, nbig = 0;
+    int nblk = 0, nsmall = 0, nbig = 0, sms = 0;
     int64_t total = 0, rows_total = 0;
     int64_t *boff = nullptr, *rot_off = nullptr;
     int *bdim = nullptr, *counters = nullptr;
@@ -308,7 +315,7 @@ struct ProjectPlan {
     // cluster jobs with their tile lists, device-resident
     struct BJStep {
         size_t o_jobs = 0, o_mem = 0, o_tiles = 0;
-        int njobs = 0, ntiles = 0;
+        int njobs = 0, ntiles = 0, kmax = 0;
     };
     std::vector<BJStep> bj_steps;
     std::vector<int> bj_nsteps;   // steps per sweep of each block (0: not scheduled)
@@ -570,9 +577,9 @@ struct ProjectPlan {
         classify_smem = (size_t)maxn * sizeof(double);
         if (classify_smem > 48 * 1024)
             V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::refine_classify_kernel, (int)classify_smem));
-        const int kc = v2b::kRefineSmallCluster;
-        V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::cluster_eig_kernel, (int)(2 * kc * (kc + 1) * sizeof(double))));
-        V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::bj_apply_kernel, (int)(3 * kc * (kc + 1) * sizeof(double))));
+        V2B_CK(v2b::prepare_cluster_eig());
+        sms = sm_count();
+        V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::bj_apply_kernel, v2b::kBjApplySmem));
         // clusters of kRefineSmallCluster+1 .. kJacobiMaxDim rows use jacobi_warm_kernel
         mid_smem = v2b::jacobi_smem_bytes(v2b::kJacobiMaxDim);
         V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::jacobi_warm_kernel, (int)std::max(smem, mid_smem)));
@@ -733,6 +740,7 @@ struct ProjectPlan {
             }
             BJStep &bs = bj_steps[st];
             bs.njobs = (int)jl.size();
+            for (const ClusterJob &j : jl) bs.kmax = std::max(bs.kmax, j.k);
             bs.ntiles = (int)tl.size();
             bs.o_jobs = sect(jl.data(), jl.size() * sizeof(ClusterJob));
             bs.o_mem = sect(ml.data(), ml.size() * 4);
@@ -755,16 +763,14 @@ struct ProjectPlan {
         if (S == 0) return;
         V2B_CK(cudaMemcpyAsync(bj_on, h_bjon, nblk * sizeof(int), cudaMemcpyHostToDevice, s));
         refine_bj_sweeps++;
-        const int kc = kRefineSmallCluster;
         for (int i = 0; i < S; i++) {
             const BJStep &bs = bj_steps[i];
             if (bs.njobs == 0) continue;
             const ClusterJob *jobs = (const ClusterJob *)(bj_dev + bs.o_jobs);
             const int *mem = (const int *)(bj_dev + bs.o_mem);
-            cluster_eig_kernel<<<bs.njobs, 256, 2 * kc * (kc + 1) * sizeof(double), s>>>(T, boff, bdim, jobs,
-                                                                                      mem, Qt, lam, bj_on,
-                                                                                      kBJInnerSweeps);
-            bj_apply_kernel<<<bs.ntiles, 256, 3 * kc * (kc + 1) * sizeof(double), s>>>(
+            V2B_CK(launch_cluster_eig(bs.njobs, bs.kmax, sms, s, T, boff, bdim, jobs, mem, Qt, lam, bj_on,
+                                      kBJInnerSweeps));
+            bj_apply_kernel<<<bs.ntiles, 256, kBjApplySmem, s>>>(
                 T, Vt, boff, bdim, jobs, mem, Qt, (const int4 *)(bj_dev + bs.o_tiles), bj_on);
             V2B_CK(cudaGetLastError());
             launches += 2;
@@ -828,7 +834,7 @@ struct ProjectPlan {
         std::vector<int> base(nblk, 0);
         for (int b = 1; b < nblk; b++) base[b] = base[b - 1] + dims[b - 1];
         int64_t qoff = 0, roff = 0;
-        int nsm = 0, nmid = 0, nbg = 0, kmax_big = 0;
+        int nsm = 0, nmid = 0, nbg = 0, kmax_small = 0, kmax_big = 0;
         for (int q = 0; q < nj_all; q++) {
             const auto &c = members[order[q]];
             ClusterJob &j = jl[q];
@@ -850,6 +856,7 @@ struct ProjectPlan {
             for (int a = 0; a < ntc; a++) tcommit.push_back(make_int4(q, a, 0, 0));
             const int kind = cls(order[q]);
             if (kind == 0) {
+                kmax_small = std::max(kmax_small, j.k);
                 nsm++;
                 continue;
             }
@@ -905,11 +912,8 @@ struct ProjectPlan {
         const int64_t *d_cb = (const int64_t *)(arena + o_cb), *d_cr = (const int64_t *)(arena + o_cr);
         const int *d_cd = (const int *)(arena + o_cd);
         if (nsm) {
-            const int kc = kRefineSmallCluster;
-            cluster_eig_kernel<<<nsm, 256, 2 * kc * (kc + 1) * sizeof(double), s>>>(T, boff, bdim, d_jobs,
-                                                                                 d_mem, Qt, lam, nullptr,
-                                                                                 kClusterSweeps);
-            V2B_CK(cudaGetLastError());
+            V2B_CK(launch_cluster_eig(nsm, kmax_small, sms, s, T, boff, bdim, d_jobs, d_mem, Qt, lam, nullptr,
+                                      kClusterSweeps));
             launches++;
         }
         if (nmid + nbg) {
@@ -1234,13 +1238,6 @@ struct ProjectPlan {
     }
 };
 
-int sm_count() {
-    int dev = 0, n = 0;
-    V2B_CK(cudaGetDevice(&dev));
-    V2B_CK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    return n;
-}
-
 }  // namespace
 
 void v2b::set_last_error(const std::string &msg) { g_last_error = msg; }
@@ -1357,7 +1354,6 @@ struct v2b_problem {
         b = dalloc<double>(nd); y = dalloc<double>(nd); Ax = dalloc<double>(nd);
         Acz = dalloc<double>(nd);
         y1 = dalloc<double>(nd); y2 = dalloc<double>(nd);
-        cg.build(hostA, hostAT, sm_count());
         stats_partials = dalloc<double>(4 * v2b::kStatsBlocks);
         cg_out = dalloc<double>(2);
         stats = dalloc<double>(4);
@@ -1371,6 +1367,9 @@ struct v2b_problem {
 
     void ensure_plan() {
         if (!plan.built) plan.build(prob.dims);
+    }
+    void ensure_cg() {   // only a solve needs the CG kernel's tables
+        if (!cg.grid) cg.build(hostA, hostAT, sm_count());
     }
 
     int grid_for(int64_t rows, int threads) const {
@@ -1492,6 +1491,7 @@ struct v2b_problem {
         check_inputs_finite();
         const int64_t np = prob.n_primal, nd = prob.n_dual;
         ensure_plan();
+        ensure_cg();
         if (keep_state) {   // continue where the last device solve stopped
             keep_state = false;
         } else if (resume) {   // mu was set with the state

@@ -107,3 +107,28 @@ def test_mixed_precision_projection_mode_matches_fp64(cuda_device):
     assert abs(e["mixed"] - e["refine"]) <= 1e-6
     assert p.refine_counts()["fp32_eigensolves"] > 0
     p.set_projection_mode("refine")
+
+
+@pytest.mark.parametrize("n,na,nb", [(5, 3, 2), (7, 4, 4), (9, 5, 4)])
+def test_block_jacobi_on_ragged_blocks(cuda_device, n, na, nb):
+    """Cold projections take block-Jacobi steps over 32-row groups: blocks of
+    25, 50, 21, 49, 98, 36, 81 and 162 rows end in groups of 1 to 31 rows, odd
+    pairs and an odd group count; clusters of equal eigenvalues and exact
+    zeros keep pairs that never rotate."""
+    import torch
+    p = hb.V2RDMProblem(n, na, nb)
+    rng = np.random.default_rng(n)
+    U = []
+    for d in (int(v) for v in p.dims):
+        q = np.linalg.qr(rng.standard_normal((d, d)))[0]
+        lam = rng.uniform(-2.0, 2.0, d)
+        lam[: d // 3] = 1.0
+        lam[d // 3: d // 2] = 0.0
+        U.append(((q * lam) @ q.T).ravel())
+    U = np.concatenate(U)
+    xr, zr = project_blocks(U, p.dims, 0.8)
+    for _ in range(2):
+        x, z = p.project(torch.from_numpy(U).to(cuda_device), 0.8)
+        scale = max(1.0, np.linalg.norm(U))
+        assert np.max(np.abs(x.cpu().numpy() - xr)) <= TOL * scale
+        assert np.max(np.abs(z.cpu().numpy() - zr)) <= TOL * scale

@@ -25,8 +25,8 @@ namespace v2b {
 //
 // FP64 tensor cores (mma.sync m8n8k4 .f64): a 64 x 64 output tile per CTA of
 // 4 warps, each warp a 32 x 32 sub-tile of 4 x 4 m8n8 fragments (32
-// accumulators per thread).  K runs in chunks of 16 through a 3-stage
-// cp.async pipeline (8-byte copies: a block of odd dimension starts at an
+// accumulators per thread).  K runs in chunks of 16 through a cp.async
+// pipeline of three stages (8-byte copies: a block of odd dimension starts at an
 // odd double, so 16-byte alignment is not available; out-of-range elements
 // are zero-filled by the copy itself).  Each operand tile is stored with its
 // global contiguous index innermost (k-major when the matrix is read down
@@ -40,18 +40,26 @@ namespace v2b {
 //
 // Split K: when a launch has fewer tiles than the grid has CTA slots, the
 // plan cuts the K range of the large blocks' tiles into S parts (tile word w:
-// bit 0 mirror, bits 4-7 the part s, bits 8-11 S, bits 12+ the output tile's
+// bit 0 mirror, bit 1 only the upper half of a diagonal tile, bits 4-7 the part s, bits 8-11 S, bits 12+ the output tile's
 // group; S <= kGemmMaxSplit).  Each part stores its 64 x 64 partial product
 // in the group's slot s of split_ws and counts itself in split_cnt[group]; the part that arrives
 // last sums the slots in the order s = 0 .. S-1 (the same bits whichever
 // part arrives last), re-arms the counter and runs the epilogue.
+//
+// Tile size: 64 x 64 tiles reuse their operands twice as often, 32 x 32 tiles
+// (a quarter of the work, 0.14 us of MMAs per K chunk against 0.54) give four
+// times as many CTAs and finish sooner where 64 x 64 tiles leave SMs idle.
 constexpr int kGemmBK = 16;
-constexpr int kGemmStages = 3;
 constexpr int kGemmThreads = 128;
-constexpr int kPadM = kGemmTile + 4;    // k-major rows: 64 + 4 doubles
 constexpr int kPadK = kGemmBK + 4;      // m-major rows: 16 + 4 doubles
-constexpr int kOpDoubles = (kGemmTile * kPadK > kGemmBK * kPadM) ? kGemmTile * kPadK : kGemmBK * kPadM;
-constexpr int kGemmSmem = kGemmStages * 2 * kOpDoubles * (int)sizeof(double);
+template <int TM>
+struct GemmShape {
+    static constexpr int kPadM = TM + 4;   // k-major rows
+    static constexpr int kOpDoubles = (TM * kPadK > kGemmBK * kPadM) ? TM * kPadK : kGemmBK * kPadM;
+    // the K chunks of a 32-row tile are short: more of them in flight
+    static constexpr int kStages = TM == 64 ? 3 : 6;
+    static constexpr int kSmem = kStages * 2 * kOpDoubles * (int)sizeof(double);
+};
 
 __device__ __forceinline__ void cp_async8(double *smem, const double *gmem, bool pred) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -73,35 +81,35 @@ __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, dou
                  : "d"(a), "d"(b));
 }
 
-// shared-memory index of element (m, k) of a 64 x 16 operand tile
-template <bool KMAJOR>
+// shared-memory index of element (m, k) of a TM x 16 operand tile
+template <int TM, bool KMAJOR>
 __device__ __forceinline__ int op_idx(int m, int k) {
-    return KMAJOR ? k * kPadM + m : m * kPadK + k;
+    return KMAJOR ? k * GemmShape<TM>::kPadM + m : m * kPadK + k;
 }
 
-// one 64 x 16 operand tile: rows m of the operand (rows of op(A) or columns of
+// one TM x 16 operand tile: rows m of the operand (rows of op(A) or columns of
 // op(B)) from m0, k from k0.  KMAJOR: the global matrix is contiguous in m
 // (element (m, k) at X[k n + m]), else in k (X[m n + k]).
-template <bool KMAJOR>
+template <int TM, bool KMAJOR>
 __device__ __forceinline__ void load_op(double *sm, const double *__restrict__ X, int n, int m0, int k0) {
 #pragma unroll
-    for (int it = 0; it < kGemmTile * kGemmBK / kGemmThreads; it++) {
+    for (int it = 0; it < TM * kGemmBK / kGemmThreads; it++) {
         const int e = it * kGemmThreads + threadIdx.x;
-        const int m = KMAJOR ? e % kGemmTile : e / kGemmBK;
-        const int k = KMAJOR ? e / kGemmTile : e % kGemmBK;
+        const int m = KMAJOR ? e % TM : e / kGemmBK;
+        const int k = KMAJOR ? e / TM : e % kGemmBK;
         const int gm = m0 + m, gk = k0 + k;
         const bool ok = gm < n && gk < n;
         const double *src = ok ? (KMAJOR ? X + (int64_t)gk * n + gm : X + (int64_t)gm * n + gk) : X;
-        cp_async8(sm + op_idx<KMAJOR>(m, k), src, ok);
+        cp_async8(sm + op_idx<TM, KMAJOR>(m, k), src, ok);
     }
 }
 
-template <bool TA, bool TB, int EPI>
+template <int TM, bool TA, bool TB, int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 3)
     gemm_tiles_kernel(const double *__restrict__ A, const double *__restrict__ B,
                       double *__restrict__ C, const int4 *__restrict__ tiles,
                       const int64_t *__restrict__ boff, const int *__restrict__ bdim,
-                      const double *__restrict__ Cin, const double *__restrict__ Us, double inv_mu,
+                      const double *__restrict__ Cin, const double *__restrict__ Us, double inv_mu, double beta,
                       double *__restrict__ xo, double *__restrict__ zo,
                       const int *__restrict__ bstate, unsigned long long *__restrict__ orth,
                       int ntiles, int *__restrict__ sched, double *__restrict__ split_ws,
@@ -109,10 +117,12 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     // op(A) rows are m-contiguous in memory when A is read transposed;
     // op(B) columns are m-contiguous when B is read as stored
     constexpr bool AK = TA, BKM = !TB;
+    constexpr int kGemmStages = GemmShape<TM>::kStages;
+    constexpr int kOpDoubles = GemmShape<TM>::kOpDoubles, F = TM / 16;   // F x F fragments per warp
     extern __shared__ double gsm[];
     __shared__ int s_tile, s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int wm = (warp >> 1) * (TM / 2), wn = (warp & 1) * (TM / 2);
     const int fr = lane >> 2, fk = lane & 3;
     for (int iter = 0;; iter++) {
         int ti;
@@ -140,13 +150,13 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
         const int blk = t.x, n = bdim[blk];
         if (bstate && bstate[blk] != 0) continue;   // uniform over the CTA
         const int64_t off = boff[blk];
-        const int r0 = t.y * kGemmTile, c0 = t.z * kGemmTile;
+        const int r0 = t.y * TM, c0 = t.z * TM;
         const double *Ab = A + off, *Bb = B + off;
-        double acc[4][4][2];
+        double acc[F][F][2];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < F; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+            for (int j = 0; j < F; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
         const int split = (t.w >> 8) & 15, part = (t.w >> 4) & 15;
         const int nk_all = (n + kGemmBK - 1) / kGemmBK;
@@ -158,8 +168,8 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
         for (int st = 0; st < kGemmStages - 1; st++) {
             if (st < nk) {
                 double *sa = gsm + st * 2 * kOpDoubles;
-                load_op<AK>(sa, Ab, n, r0, (kb + st) * kGemmBK);
-                load_op<BKM>(sa + kOpDoubles, Bb, n, c0, (kb + st) * kGemmBK);
+                load_op<TM, AK>(sa, Ab, n, r0, (kb + st) * kGemmBK);
+                load_op<TM, BKM>(sa + kOpDoubles, Bb, n, c0, (kb + st) * kGemmBK);
             }
             cp_async_commit();
         }
@@ -170,23 +180,23 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
             const int kn = kt + kGemmStages - 1;
             if (kn < nk) {
                 double *sa = gsm + (kn % kGemmStages) * 2 * kOpDoubles;
-                load_op<AK>(sa, Ab, n, r0, (kb + kn) * kGemmBK);
-                load_op<BKM>(sa + kOpDoubles, Bb, n, c0, (kb + kn) * kGemmBK);
+                load_op<TM, AK>(sa, Ab, n, r0, (kb + kn) * kGemmBK);
+                load_op<TM, BKM>(sa + kOpDoubles, Bb, n, c0, (kb + kn) * kGemmBK);
             }
             cp_async_commit();
             const double *sa = gsm + (kt % kGemmStages) * 2 * kOpDoubles;
             const double *sb = sa + kOpDoubles;
 #pragma unroll
             for (int k4 = 0; k4 < kGemmBK; k4 += 4) {
-                double a[4], b[4];
+                double a[F], b[F];
 #pragma unroll
-                for (int i = 0; i < 4; i++) a[i] = sa[op_idx<AK>(wm + i * 8 + fr, k4 + fk)];
+                for (int i = 0; i < F; i++) a[i] = sa[op_idx<TM, AK>(wm + i * 8 + fr, k4 + fk)];
 #pragma unroll
-                for (int j = 0; j < 4; j++) b[j] = sb[op_idx<BKM>(wn + j * 8 + fr, k4 + fk)];
+                for (int j = 0; j < F; j++) b[j] = sb[op_idx<TM, BKM>(wn + j * 8 + fr, k4 + fk)];
 #pragma unroll
-                for (int i = 0; i < 4; i++)
+                for (int i = 0; i < F; i++)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+                    for (int j = 0; j < F; j++) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
             }
         }
         cp_async_wait<0>();
@@ -194,30 +204,30 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
 
         if (split > 1) {
             const unsigned group = (unsigned)t.w >> 12;
-            double *slot = split_ws + ((int64_t)group * kGemmMaxSplit + part) * (kGemmTile * kGemmTile);
+            double *slot = split_ws + ((int64_t)group * kGemmMaxSplit + part) * (TM * TM);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < F; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++)
+                for (int j = 0; j < F; j++)
 #pragma unroll
                     for (int h = 0; h < 2; h++)
-                        __stcg(slot + (wm + i * 8 + fr) * kGemmTile + wn + j * 8 + 2 * fk + h, acc[i][j][h]);
+                        __stcg(slot + (wm + i * 8 + fr) * TM + wn + j * 8 + 2 * fk + h, acc[i][j][h]);
             __threadfence();
             __syncthreads();
             if (threadIdx.x == 0) s_last = atomicAdd(split_cnt + group, 1) == split - 1;
             __syncthreads();
             if (!s_last) continue;
             __threadfence();
-            const double *slots = split_ws + (int64_t)group * kGemmMaxSplit * (kGemmTile * kGemmTile);
+            const double *slots = split_ws + (int64_t)group * kGemmMaxSplit * (TM * TM);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < F; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++)
+                for (int j = 0; j < F; j++)
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        const int e = (wm + i * 8 + fr) * kGemmTile + wn + j * 8 + 2 * fk + h;
+                        const int e = (wm + i * 8 + fr) * TM + wn + j * 8 + 2 * fk + h;
                         double v = __ldcg(slots + e);
-                        for (int q = 1; q < split; q++) v += __ldcg(slots + q * (kGemmTile * kGemmTile) + e);
+                        for (int q = 1; q < split; q++) v += __ldcg(slots + q * (TM * TM) + e);
                         acc[i][j][h] = v;
                     }
             if (threadIdx.x == 0) split_cnt[group] = 0;   // every part has arrived: re-arm
@@ -225,15 +235,16 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
 
         double dev = 0.0;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < F; i++) {
             const int r = r0 + wm + i * 8 + fr;
             if (r >= n) continue;
 #pragma unroll
-            for (int j = 0; j < 4; j++)
+            for (int j = 0; j < F; j++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int c = c0 + wn + j * 8 + 2 * fk + h;
                     if (c >= n) continue;
+                    if ((t.w & 2) && c < r) continue;   // a strictly symmetric result's diagonal tile
                     const double v = acc[i][j][h];
                     // t.w: an off-diagonal tile of a symmetric product, stored
                     // at (r, c) and at its mirror image (c, r)
@@ -247,6 +258,12 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
                             const double id = (r == c) ? 1.0 : 0.0;
                             C[e] = 1.5 * id - 0.5 * v;
                             dev = fmax(dev, fabs(v - id));
+                        } else if (EPI == kEpiLinear) {
+                            C[e] = inv_mu * Cin[e] + beta * v;
+                        } else if (EPI == kEpiSign) {   // v = Us sign(Us)
+                            const double up = 0.5 * (Us[e] + v);
+                            xo[e] = up * inv_mu;
+                            zo[e] = up - Us[e];
                         } else {   // kEpiProject: v = U+
                             xo[e] = v * inv_mu;
                             zo[e] = v - Us[e];
@@ -263,10 +280,11 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     }
 }
 
-template <bool TA, bool TB, int EPI>
+template <int TM, bool TA, bool TB, int EPI>
 static cudaError_t launch_variant(int ntiles, cudaStream_t s, GEMM_ARGS, int *sched, double *split_ws,
-                                  int *split_cnt) {
-    auto kern = gemm_tiles_kernel<TA, TB, EPI>;
+                                  int *split_cnt, double beta) {
+    auto kern = gemm_tiles_kernel<TM, TA, TB, EPI>;
+    constexpr int kGemmSmem = GemmShape<TM>::kSmem;
     // opt in to the pipeline's shared memory and size the persistent grid,
     // once per variant, device and context (function attributes are per
     // device and do not survive a cudaDeviceReset)
@@ -299,29 +317,20 @@ static cudaError_t launch_variant(int ntiles, cudaStream_t s, GEMM_ARGS, int *sc
         cfg = cache[dev];
     }
     const int grid = sched ? std::min(ntiles, cfg.slots) : ntiles;
-    kern<<<grid, kGemmThreads, kGemmSmem, s>>>(A, B, C, tiles, boff, bdim, Cin, Us, inv_mu, xo, zo, bstate,
-                                               orth, ntiles, sched, split_ws, split_cnt);
+    kern<<<grid, kGemmThreads, kGemmSmem, s>>>(A, B, C, tiles, boff, bdim, Cin, Us, inv_mu, beta, xo, zo,
+                                               bstate, orth, ntiles, sched, split_ws, split_cnt);
     return cudaGetLastError();
 }
 
-cudaError_t gemm_slots(int *slots) {
-    int dev = 0, sms = 0, occ = 0;
-    const void *kern = (const void *)gemm_tiles_kernel<false, false, kEpiStore>;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = raise_dynamic_smem(kern, kGemmSmem);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kGemmThreads, kGemmSmem);
-    if (e == cudaSuccess) *slots = std::max(1, sms * occ);
-    return e;
-}
-
 cudaError_t launch_gemm_tiles(GemmVariant v, int ntiles, cudaStream_t s, GEMM_ARGS, int *sched, double *split_ws,
-                              int *split_cnt) {
+                              int *split_cnt, int tile, double beta) {
     if (ntiles <= 0) return cudaSuccess;
-#define V2B_GEMM_CASE(NAME, TA, TB, EPI) \
-    case NAME:                           \
-        return launch_variant<TA, TB, EPI>(ntiles, s, A, B, C, tiles, boff, bdim, Cin, Us, inv_mu, xo, zo, bstate, orth, \
-                                           sched, split_ws, split_cnt);
+#define V2B_GEMM_CASE(NAME, TA, TB, EPI)                                                                            \
+    case NAME:                                                                                                      \
+        return tile == 32 ? launch_variant<32, TA, TB, EPI>(ntiles, s, A, B, C, tiles, boff, bdim, Cin, Us, inv_mu, \
+                                                            xo, zo, bstate, orth, sched, split_ws, split_cnt, beta)  \
+                          : launch_variant<64, TA, TB, EPI>(ntiles, s, A, B, C, tiles, boff, bdim, Cin, Us, inv_mu, \
+                                                            xo, zo, bstate, orth, sched, split_ws, split_cnt, beta);
     switch (v) {
         V2B_GEMM_CASE(kGemmNTNewtonSchulz, false, true, kEpiNS)
         V2B_GEMM_CASE(kGemmNTStore, false, true, kEpiStore)
@@ -329,6 +338,8 @@ cudaError_t launch_gemm_tiles(GemmVariant v, int ntiles, cudaStream_t s, GEMM_AR
         V2B_GEMM_CASE(kGemmTNStore, true, false, kEpiStore)
         V2B_GEMM_CASE(kGemmNNProject, false, false, kEpiProject)
         V2B_GEMM_CASE(kGemmNNAdd, false, false, kEpiAdd)
+        V2B_GEMM_CASE(kGemmNTLinear, false, true, kEpiLinear)
+        V2B_GEMM_CASE(kGemmNTSign, false, true, kEpiSign)
     }
 #undef V2B_GEMM_CASE
     return cudaErrorInvalidValue;

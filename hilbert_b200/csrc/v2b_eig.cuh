@@ -12,6 +12,8 @@ constexpr int kEpiStore = 0;     // C = op(A) op(B)
 constexpr int kEpiAdd = 1;       // C = Cin + op(A) op(B)
 constexpr int kEpiProject = 2;   // x = (op(A) op(B)) / mu, z = op(A) op(B) - Us
 constexpr int kEpiNS = 3;        // C = 3/2 I - 1/2 op(A) op(B); orth[b] = max |op(A) op(B) - I|
+constexpr int kEpiLinear = 4;    // C = inv_mu Cin + beta op(A) op(B)
+constexpr int kEpiSign = 5;      // U+ = (Us + op(A) op(B)) / 2: x = U+ / mu, z = U+ - Us
 constexpr int kGemmTile = 64;
 constexpr int kGemmMaxSplit = 4;   // K parts of one output tile at most
 
@@ -32,15 +34,13 @@ constexpr int kGemmMaxSplit = 4;   // K parts of one output tile at most
 // zero again); null launches one CTA per tile.  Launches that share a sched
 // pair must be ordered (one stream).  Tiles split along K (tile word bits
 // 8-11 above 1) need split_ws (kGemmMaxSplit x 64 x 64 doubles per group) and split_cnt
-// (one int per group, zero before the first launch, left zero).
+// (one int per group, zero before the first launch, left zero).  tile: 64 or
+// 32, the tile size that the list counts in.
 enum GemmVariant { kGemmNTStore = 0, kGemmNNStore = 1, kGemmTNStore = 2, kGemmNNProject = 3,
-                   kGemmNNAdd = 4, kGemmNTNewtonSchulz = 5 };
+                   kGemmNNAdd = 4, kGemmNTNewtonSchulz = 5, kGemmNTLinear = 6, kGemmNTSign = 7 };
 cudaError_t launch_gemm_tiles(GemmVariant v, int ntiles, cudaStream_t s, GEMM_ARGS,
-                              int *sched = nullptr, double *split_ws = nullptr, int *split_cnt = nullptr);
-// CTA slots of the persistent GEMM grid on the current device (SMs x
-// resident CTAs)
-cudaError_t gemm_slots(int *slots);
-
+                              int *sched = nullptr, double *split_ws = nullptr, int *split_cnt = nullptr,
+                              int tile = kGemmTile, double beta = 0.0);
 }  // namespace v2b
 
 #include <string>

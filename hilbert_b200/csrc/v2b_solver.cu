@@ -27,6 +27,7 @@
 #include "v2b_kernels.cuh"
 #include "v2b_orbital.cuh"
 #include "v2b_refine.cuh"
+#include "v2b_sign.cuh"
 #include "cg_tables.h"
 #include "v2rdm_b200.h"
 #include "v2rdm_problem.h"
@@ -265,6 +266,12 @@ struct ProjectPlan {
     static constexpr int kSplitMinDim = 256;
     int4 *ktiles = nullptr, *kstiles = nullptr;
     int nktiles = 0, nkstiles = 0;
+    // The GEMMs' tile size.  32 where the 64 x 64 tiles would leave SMs idle,
+    // if no block has tiles to cut along K: 9.1 us a launch against 22.6 for
+    // the blocks of 45 to 200 rows of (10e,10o).
+    int gtile = v2b::kGemmTile;
+    int4 *gtiles = nullptr;   // the full list in that size (the elementwise kernels keep 64)
+    int ngtiles = 0;
     double *split_ws = nullptr;
     int *split_cnt = nullptr;
     bool split_k = true;
@@ -369,6 +376,28 @@ struct ProjectPlan {
         }
         pev_used = 0;
     }
+    // A stand-alone projection returns with its kernels still running on the
+    // caller's stream; whoever uses the work arrays next on another stream
+    // waits for them.
+    cudaEvent_t used = nullptr;
+    cudaStream_t used_on = nullptr;
+    bool used_pending = false;
+    void mark_used(cudaStream_t s) {
+        V2B_CK(cudaEventRecord(used, s));
+        used_on = s;
+        used_pending = true;
+    }
+    void wait_used(cudaStream_t s) {
+        if (!used_pending) return;
+        if (used_on != s) V2B_CK(cudaStreamWaitEvent(s, used, 0));
+    }
+    // project_once: its block lists and scaling scratch
+    int *sign_list = nullptr, *sign_state = nullptr;
+    int4 *sign_tiles = nullptr;
+    int nsign_tiles = 0;
+    double *sign_part = nullptr;
+    int nsign_small = 0, sign_small_max = 0;
+    bool sign_large = false;
     bool fresh = true;
     bool built = false;
     // 0: warm refinement; 1: selective Jacobi on every block, every call;
@@ -411,7 +440,7 @@ struct ProjectPlan {
     // T = Vt W (symmetric list).
     void tune_split(const std::vector<int> &d, const std::vector<int4> &tl, const std::vector<int4> &stl) {
         using namespace v2b;
-        int groups = 0;
+        int groups = 0;   // output tiles of blocks to cut
         split_tiles(d, tl, 2, groups);
         split_ws = dalloc<double>((size_t)std::max(groups, 1) * kGemmMaxSplit * kGemmTile * kGemmTile);
         split_cnt = dalloc<int>(std::max(groups, 1));
@@ -430,6 +459,7 @@ struct ProjectPlan {
             int best_s = 1;
             float best = 0.0f;
             for (int S : {1, 2, kGemmMaxSplit}) {
+                if (groups == 0) break;   // no block to cut: one piece
                 int g = 0;
                 const std::vector<int4> k = split_tiles(d, L, S, g);
                 if (k.empty()) break;
@@ -440,11 +470,11 @@ struct ProjectPlan {
                     if (sym)
                         V2B_CK(launch_gemm_tiles(kGemmNNStore, (int)k.size(), s, Vt, W, T, buf, boff, bdim, nullptr,
                                                  Us, 0.0, nullptr, nullptr, nullptr, orth, gemm_sched, split_ws,
-                                                 split_cnt));
+                                                 split_cnt, gtile));
                     else
                         V2B_CK(launch_gemm_tiles(kGemmNTStore, (int)k.size(), s, Us, Vt, W, buf, boff, bdim, nullptr,
                                                  Us, 0.0, nullptr, nullptr, nullptr, orth, gemm_sched, split_ws,
-                                                 split_cnt));
+                                                 split_cnt, gtile));
                 }
                 V2B_CK(cudaEventRecord(e1, s));
                 V2B_CK(cudaEventSynchronize(e1));
@@ -515,9 +545,27 @@ struct ProjectPlan {
         // longest K first: the persistent GEMM grid takes tiles in this order
         std::stable_sort(tl.begin(), tl.end(), [&](const int4 &a, const int4 &b) { return d[a.x] > d[b.x]; });
         ntiles = (int)tl.size();
+        sms = sm_count();
+        gtile = maxn < kSplitMinDim && ntiles <= sms ? 32 : v2b::kGemmTile;
+        std::vector<int4> gtl = tl;
+        if (gtile == 32) {
+            gtl.clear();
+            for (int i = 0; i < nblk; i++) {
+                const int nt = (d[i] + 31) / 32;
+                for (int a = 0; a < nt; a++)
+                    for (int b = 0; b < nt; b++) gtl.push_back(make_int4(i, a, b, 0));
+            }
+            std::stable_sort(gtl.begin(), gtl.end(), [&](const int4 &a, const int4 &b) { return d[a.x] > d[b.x]; });
+        }
+        ngtiles = (int)gtl.size();
+        gtiles = dalloc<int4>(std::max(ngtiles, 1));
+        if (ngtiles) V2B_CK(cudaMemcpy(gtiles, gtl.data(), ngtiles * sizeof(int4), cudaMemcpyHostToDevice));
         std::vector<int4> stl;
-        for (const int4 &t : tl)
-            if (t.y <= t.z) stl.push_back(make_int4(t.x, t.y, t.z, t.y < t.z ? 1 : 0));
+        // (32-row tiles: the four of a 64-row diagonal tile are all computed, as
+        // one 64-row tile computes them, so that the tile size leaves no trace)
+        const int h = v2b::kGemmTile / gtile;
+        for (const int4 &t : gtl)
+            if (t.y / h <= t.z / h) stl.push_back(make_int4(t.x, t.y, t.z, t.y / h < t.z / h ? 1 : 0));
         nstiles = (int)stl.size();
         stiles = dalloc<int4>(std::max(nstiles, 1));
         if (nstiles) V2B_CK(cudaMemcpy(stiles, stl.data(), nstiles * sizeof(int4), cudaMemcpyHostToDevice));
@@ -532,7 +580,7 @@ struct ProjectPlan {
         V2B_CK(cudaMemcpy(bdim, d.data(), nblk * 4, cudaMemcpyHostToDevice));
         V2B_CK(cudaMemset(counters, 0, 16));
         if (ntiles) V2B_CK(cudaMemcpy(tiles, tl.data(), ntiles * sizeof(int4), cudaMemcpyHostToDevice));
-        tune_split(d, tl, stl);
+        tune_split(d, gtl, stl);
         if (nsmall) rot = dalloc<double2>(ro);
         if (smem)
             V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::jacobi_warm_kernel, (int)smem));
@@ -578,13 +626,13 @@ struct ProjectPlan {
         if (classify_smem > 48 * 1024)
             V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::refine_classify_kernel, (int)classify_smem));
         V2B_CK(v2b::prepare_cluster_eig());
-        sms = sm_count();
         V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::bj_apply_kernel, v2b::kBjApplySmem));
         // clusters of kRefineSmallCluster+1 .. kJacobiMaxDim rows use jacobi_warm_kernel
         mid_smem = v2b::jacobi_smem_bytes(v2b::kJacobiMaxDim);
         V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::jacobi_warm_kernel, (int)std::max(smem, mid_smem)));
         build_block_jacobi();
         V2B_CK(cudaEventCreateWithFlags(&staged, cudaEventDisableTiming));
+        V2B_CK(cudaEventCreateWithFlags(&used, cudaEventDisableTiming));
         fresh = true;
         built = true;
     }
@@ -593,9 +641,12 @@ struct ProjectPlan {
         for (auto e : pev) cudaEventDestroy(e);
         pev.clear();
         if (staged) cudaEventDestroy(staged);
+        if (used) cudaEventDestroy(used);
+        used = nullptr;
+        used_pending = false;
         staged = nullptr;
         staged_pending = false;
-        for (void *q : {(void *)boff, (void *)rot_off, (void *)bdim, (void *)counters, (void *)tiles, (void *)stiles,
+        for (void *q : {(void *)boff, (void *)rot_off, (void *)bdim, (void *)counters, (void *)tiles, (void *)stiles, (void *)gtiles,
                         (void *)ktiles, (void *)kstiles, (void *)split_ws, (void *)split_cnt, (void *)gemm_sched, (void *)rot, (void *)Vt, (void *)Vt2, (void *)Us, (void *)W, (void *)T,
                         (void *)P, (void *)rec_b, (void *)norm_b, (void *)sub_boff, (void *)sub_roff,
                         (void *)sub_bdim, (void *)bstate, (void *)orth, (void *)bnorm, (void *)norm_part,
@@ -603,9 +654,14 @@ struct ProjectPlan {
                         (void *)Tsave, (void *)arena, (void *)crec, (void *)cnorm, (void *)Tc,
                         (void *)Pc, (void *)bj_dev, (void *)bj_on,
                         (void *)rowbase, (void *)lam, (void *)Qt, (void *)sub32_boff, (void *)sub32_roff,
-                        (void *)sub32_bdim, (void *)T32})
+                        (void *)sub32_bdim, (void *)T32, (void *)sign_list, (void *)sign_state, (void *)sign_part, (void *)sign_tiles})
             cudaFree(q);
         T32 = nullptr;
+        sign_list = sign_state = nullptr;
+        sign_tiles = nullptr;
+        sign_part = nullptr;
+        sign_small_max = 0;
+        sign_large = false;
         for (void *q : {(void *)h_sub, (void *)h_bstate_up, (void *)h_state, (void *)h_edges,
                         (void *)h_arena, (void *)h_bjon})
             if (q) cudaFreeHost(q);
@@ -618,10 +674,10 @@ struct ProjectPlan {
               double inv_mu, double *x, double *z, cudaStream_t s, long &launches,
               const int *only_work = nullptr, bool sym = false) {
         ph_begin(0, s);
-        const int nt = sym ? (split_k ? nkstiles : nstiles) : (split_k ? nktiles : ntiles);
-        const int4 *tl = sym ? (split_k ? kstiles : stiles) : (split_k ? ktiles : tiles);
+        const int nt = sym ? (split_k ? nkstiles : nstiles) : (split_k ? nktiles : ngtiles);
+        const int4 *tl = sym ? (split_k ? kstiles : stiles) : (split_k ? ktiles : gtiles);
         V2B_CK(v2b::launch_gemm_tiles(v, nt, s, A, B, C, tl, boff, bdim, Cin, Us, inv_mu, x, z, only_work, orth,
-                                      gemm_sched, split_ws, split_cnt));
+                                      gemm_sched, split_ws, split_cnt, gtile));
         ph_end(s);
         launches++;
     }
@@ -1197,6 +1253,71 @@ struct ProjectPlan {
         }
     }
 
+    // A projection from scratch that leaves no basis behind (mode 0): by the
+    // matrix sign function (v2b_sign.cu), small blocks in one CTA each, the
+    // larger ones through the GEMM tiles.  No host decision, no copy back.
+    void project_once(const double *U, double mu, double *x, double *z, cudaStream_t s, long &launches) {
+        using namespace v2b;
+        if (nblk == 0 || ntiles == 0) return;
+        if (!sign_list) {   // the blocks' classes, once
+            std::vector<int> small, state(nblk, 1);
+            for (int b = 0; b < nblk; b++) {
+                if (dims[b] >= 1 && dims[b] <= kSignSmallDim) {
+                    small.push_back(b);
+                    sign_small_max = std::max(sign_small_max, dims[b]);
+                } else if (dims[b] > kSignSmallDim) {
+                    state[b] = 0;
+                    sign_large = true;
+                }
+            }
+            // upper tiles, each element computed once and mirrored: the
+            // iteration amplifies an asymmetry
+            std::vector<int4> tl;
+            for (int b = 0; b < nblk; b++) {
+                if (state[b]) continue;
+                const int nt = (dims[b] + gtile - 1) / gtile;
+                for (int i = 0; i < nt; i++)
+                    for (int j = i; j < nt; j++) tl.push_back(make_int4(b, i, j, i < j ? 1 : 3));
+            }
+            std::stable_sort(tl.begin(), tl.end(), [&](const int4 &a, const int4 &b) { return dims[a.x] > dims[b.x]; });
+            nsign_tiles = (int)tl.size();
+            sign_tiles = dalloc<int4>(tl.size());
+            if (nsign_tiles)
+                V2B_CK(cudaMemcpyAsync(sign_tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+            nsign_small = (int)small.size();
+            sign_list = dalloc<int>(small.size());
+            sign_state = dalloc<int>(nblk);
+            sign_part = dalloc<double>(2 * (size_t)kSignSplit * nblk);
+            if (nsign_small) V2B_CK(cudaMemcpyAsync(sign_list, small.data(), small.size() * 4, cudaMemcpyHostToDevice, s));
+            V2B_CK(cudaMemcpyAsync(sign_state, state.data(), nblk * 4, cudaMemcpyHostToDevice, s));
+            V2B_CK(cudaStreamSynchronize(s));   // the lists are host temporaries
+        }
+        if (nsign_small) {
+            V2B_CK(launch_sign_small(nsign_small, sign_list, sign_small_max, U, boff, bdim, 1.0 / mu, x, z, s));
+            launches++;
+        }
+        if (!sign_large) return;
+        SignStep step[kSignMaxSteps];
+        const int n = sign_steps(step);
+        symmetrize_kernel<<<ntiles, 256, 0, s>>>(U, Us, tiles, boff, bdim);
+        V2B_CK(cudaGetLastError());
+        V2B_CK(launch_sign_scale(nblk, ntiles, tiles, sign_state, Us, boff, bdim, sign_part, T, s));
+        launches += 4;
+        auto product = [&](GemmVariant v, const double *A, const double *B, double *C, const double *Cin, double a,
+                           double b) {
+            V2B_CK(launch_gemm_tiles(v, nsign_tiles, s, A, B, C, sign_tiles, boff, bdim, Cin, Us, a, x, z, nullptr,
+                                     orth, gemm_sched, nullptr, nullptr, gtile, b));
+            launches++;
+        };
+        double *X = T, *X2 = P;
+        for (int k = 0; k < n; k++) {
+            product(kGemmNTStore, X, X, W, nullptr, 0.0, 0.0);
+            product(kGemmNTLinear, X, W, X2, X, step[k].a, step[k].b);
+            std::swap(X, X2);
+        }
+        product(kGemmNTSign, Us, X, nullptr, nullptr, 1.0 / mu, 0.0);
+    }
+
     void project(const double *U, double mu, double *x, double *z, cudaStream_t s, long &launches) {
         using namespace v2b;
         if (nblk == 0 || ntiles == 0) return;
@@ -1491,6 +1612,7 @@ struct v2b_problem {
         check_inputs_finite();
         const int64_t np = prob.n_primal, nd = prob.n_dual;
         ensure_plan();
+        plan.wait_used(stream);
         ensure_cg();
         if (keep_state) {   // continue where the last device solve stopped
             keep_state = false;
@@ -1850,9 +1972,15 @@ int v2b_problem_project(v2b_problem *p, const double *d_U, double mu, double *d_
         p->setup();
         p->ensure_plan();
         // a stand-alone projection has no previous basis: solve each block from scratch
+        p->plan.wait_used((cudaStream_t)stream);
         p->plan.reset();
-        p->plan.project(d_U, mu, d_x, d_z, (cudaStream_t)stream, p->launches);
-        p->plan.reset();
+        if (p->plan.mode == 0) {
+            p->plan.project_once(d_U, mu, d_x, d_z, (cudaStream_t)stream, p->launches);
+        } else {
+            p->plan.project(d_U, mu, d_x, d_z, (cudaStream_t)stream, p->launches);
+            p->plan.reset();
+        }
+        p->plan.mark_used((cudaStream_t)stream);
         return V2B_OK;
     });
 }
@@ -1863,7 +1991,9 @@ int v2b_problem_project_warm(v2b_problem *p, const double *d_U, double mu, doubl
             throw std::invalid_argument("project_warm: bad argument");
         p->setup();
         p->ensure_plan();
+        p->plan.wait_used((cudaStream_t)stream);
         p->plan.project(d_U, mu, d_x, d_z, (cudaStream_t)stream, p->launches);
+        p->plan.mark_used((cudaStream_t)stream);
         return V2B_OK;
     });
 }

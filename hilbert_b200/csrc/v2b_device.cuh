@@ -10,27 +10,6 @@ constexpr uint32_t kDevColMask = (1u << 27) - 1u;
 constexpr int kStatusTimeout = 4;   // V2B_DEVICE_TIMEOUT
 constexpr int kStatusNan = 3;       // V2B_NAN
 
-// One packed sparse row: sum of coef * x[col] in stored order, with separate
-// multiply and add roundings (no FMA contraction), so that the result equals
-// hilbert's own left-to-right accumulation.  Entries flagged with bit 31 are
-// summed into a second partial that is added at the end (rows the reference
-// assembles as "(D2 - Q2) + (sum of delta terms)", q2.cc:218-318).
-__device__ __forceinline__ double packed_row(const uint32_t *__restrict__ ent, uint32_t b,
-                                             uint32_t e, const double *__restrict__ x,
-                                             const double *pal) {
-    double acc0 = 0.0, acc1 = 0.0;
-    bool grp = false;
-#pragma unroll 4
-    for (uint32_t k = b; k < e; k++) {
-        const uint32_t w = __ldg(ent + k);
-        const double v = __dmul_rn(pal[(w >> 27) & 15u], __ldg(x + (w & kDevColMask)));
-        grp = grp || (w >> 31);
-        if (grp) acc1 = __dadd_rn(acc1, v);
-        else acc0 = __dadd_rn(acc0, v);
-    }
-    return grp ? __dadd_rn(acc0, acc1) : acc0;
-}
-
 // the GPU's nanosecond clock (PTX %globaltimer)
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;

@@ -15,58 +15,147 @@
 
 namespace v2b {
 
-__global__ void spmv_kernel(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ent,
-                            int64_t nrows, const double *__restrict__ x, double *__restrict__ y,
-                            Palette pal) {
-    __shared__ double spal[16];
-    if (threadIdx.x < 16) spal[threadIdx.x] = pal.v[threadIdx.x];
-    __syncthreads();
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows;
-         r += (int64_t)gridDim.x * blockDim.x)
-        y[r] = packed_row(ent, __ldg(rp + r), __ldg(rp + r + 1), x, spal);
-}
+// ---------------------------------------------------------------- maps
+// A x and A^T y in hilbert's order: a row's products (one multiply rounding
+// each) are added left to right, entries from the first flagged one on in a
+// second sum.  Most rows hold one to three entries, a thread each, kRowBatch
+// entries' operands in flight; the few long ones (traces, contractions: up to
+// 400 entries at (20e,20o)) would each hold a thread for as many dependent
+// additions behind loads, so they go to a warp each, first in the grid: the
+// lanes fetch and multiply 128 entries at a time, one lane per sum adds them
+// in order from shared memory.
+//
+// Measured on B200, (20e,20o), A x and A^T y together: 60 us (a thread for
+// every row: 124).
+constexpr int kRowBatch = 4;
+constexpr int kSpmvWarps = kSpmvThreads / 32;
+constexpr int kLongChunk = 128;
 
-__global__ void spmv_A2_kernel(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ent,
-                               int64_t nrows, const double *__restrict__ x,
-                               const double *__restrict__ c, const double *__restrict__ z,
-                               double *__restrict__ Ax, double *__restrict__ Acz, Palette pal) {
-    __shared__ double spal[16];
-    if (threadIdx.x < 16) spal[threadIdx.x] = pal.v[threadIdx.x];
-    __syncthreads();
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows;
-         r += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t b = __ldg(rp + r), e = __ldg(rp + r + 1);
-        double a0 = 0.0, a1 = 0.0, w0 = 0.0, w1 = 0.0;
+struct OneVector {
+    static constexpr int N = 1;
+    const double *x;
+    __device__ __forceinline__ void get(uint32_t c, double (&v)[1]) const { v[0] = __ldg(x + c); }
+};
+struct XAndCz {   // x and c - z
+    static constexpr int N = 2;
+    const double *x, *c, *z;
+    __device__ __forceinline__ void get(uint32_t k, double (&v)[2]) const {
+        v[0] = __ldg(x + k);
+        v[1] = __dsub_rn(__ldg(c + k), __ldg(z + k));
+    }
+};
+
+// out(row, sums) for every row
+template <class X, class F>
+__device__ __forceinline__ void row_sums(const SpmvRows &R, const X &x, const double *pal, F &&out) {
+    constexpr int N = X::N;
+    __shared__ double buf[kSpmvWarps][N][kLongChunk];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x < R.long_blocks) {
+        const uint32_t q = blockIdx.x * kSpmvWarps + warp;
+        if (q >= R.nlong) return;
+        const uint32_t r = __ldg(R.long_rows + q), b = __ldg(R.rp + r), e = __ldg(R.rp + r + 1);
+        double acc0 = 0.0, acc1 = 0.0;
         bool grp = false;
-        for (uint32_t k = b; k < e; k++) {
-            const uint32_t w = __ldg(ent + k);
-            const uint32_t col = w & kDevColMask;
-            const double cf = spal[(w >> 27) & 15u];
-            const double vx = __dmul_rn(cf, __ldg(x + col));
-            const double vw = __dmul_rn(cf, __dsub_rn(__ldg(c + col), __ldg(z + col)));
-            grp = grp || (w >> 31);
-            if (grp) { a1 = __dadd_rn(a1, vx); w1 = __dadd_rn(w1, vw); }
-            else { a0 = __dadd_rn(a0, vx); w0 = __dadd_rn(w0, vw); }
+        for (uint32_t k0 = b; k0 < e; k0 += kLongChunk) {
+            const int cnt = (int)min((uint32_t)kLongChunk, e - k0);
+            uint32_t w[kLongChunk / 32];
+            double v[kLongChunk / 32][N];
+#pragma unroll
+            for (int i = 0; i < kLongChunk / 32; i++) w[i] = 32 * i + lane < cnt ? __ldg(R.ent + k0 + 32 * i + lane) : 0u;
+#pragma unroll
+            for (int i = 0; i < kLongChunk / 32; i++) x.get(w[i] & kDevColMask, v[i]);
+            int first = cnt;   // the first flagged entry of the chunk
+#pragma unroll
+            for (int i = kLongChunk / 32 - 1; i >= 0; i--) {
+                const unsigned m = __ballot_sync(0xffffffffu, w[i] >> 31);
+                if (m) first = 32 * i + __ffs(m) - 1;
+#pragma unroll
+                for (int n = 0; n < N; n++) buf[warp][n][32 * i + lane] = __dmul_rn(pal[(w[i] >> 27) & 15u], v[i][n]);
+            }
+            __syncwarp();
+            if (lane < N) {
+                const int split = grp ? 0 : first;
+#pragma unroll 8
+                for (int i = 0; i < split; i++) acc0 = __dadd_rn(acc0, buf[warp][lane][i]);
+#pragma unroll 8
+                for (int i = split; i < cnt; i++) acc1 = __dadd_rn(acc1, buf[warp][lane][i]);
+            }
+            grp = grp || first < cnt;
+            __syncwarp();
         }
-        Ax[r] = grp ? __dadd_rn(a0, a1) : a0;
-        Acz[r] = grp ? __dadd_rn(w0, w1) : w0;
+        double s[N];
+        const double mine = grp ? __dadd_rn(acc0, acc1) : acc0;
+#pragma unroll
+        for (int n = 0; n < N; n++) s[n] = __shfl_sync(0xffffffffu, mine, n);
+        if (lane == 0) out((int64_t)r, s);
+        return;
+    }
+    for (int64_t r = (int64_t)(blockIdx.x - R.long_blocks) * blockDim.x + threadIdx.x; r < R.nrows;
+         r += (int64_t)(gridDim.x - R.long_blocks) * blockDim.x) {
+        const uint32_t b = __ldg(R.rp + r), e = __ldg(R.rp + r + 1);
+        if (e - b > kSpmvLongRow) continue;
+        double acc0[N] = {}, acc1[N] = {};
+        bool grp = false;
+        for (uint32_t k0 = b; k0 < e; k0 += kRowBatch) {
+            uint32_t w[kRowBatch];
+            double v[kRowBatch][N];
+#pragma unroll
+            for (int i = 0; i < kRowBatch; i++) w[i] = k0 + i < e ? __ldg(R.ent + k0 + i) : 0u;
+#pragma unroll
+            for (int i = 0; i < kRowBatch; i++)
+                if (k0 + i < e) x.get(w[i] & kDevColMask, v[i]);
+#pragma unroll
+            for (int i = 0; i < kRowBatch; i++) {
+                if (k0 + i >= e) continue;
+                grp = grp || (w[i] >> 31);
+#pragma unroll
+                for (int n = 0; n < N; n++) {
+                    const double u = __dmul_rn(pal[(w[i] >> 27) & 15u], v[i][n]);
+                    if (grp) acc1[n] = __dadd_rn(acc1[n], u);
+                    else acc0[n] = __dadd_rn(acc0[n], u);
+                }
+            }
+        }
+        double s[N];
+#pragma unroll
+        for (int n = 0; n < N; n++) s[n] = grp ? __dadd_rn(acc0[n], acc1[n]) : acc0[n];
+        out(r, s);
     }
 }
 
-__global__ void spmv_AT_U_kernel(const uint32_t *__restrict__ rp,
-                                 const uint32_t *__restrict__ ent, int64_t nrows,
-                                 const double *__restrict__ y, const double *__restrict__ x,
-                                 const double *__restrict__ c, double mu,
-                                 double *__restrict__ ATy, double *__restrict__ U, Palette pal) {
+__global__ void __launch_bounds__(kSpmvThreads)
+    spmv_kernel(SpmvRows R, const double *__restrict__ x, double *__restrict__ y, Palette pal) {
     __shared__ double spal[16];
     if (threadIdx.x < 16) spal[threadIdx.x] = pal.v[threadIdx.x];
     __syncthreads();
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows;
-         r += (int64_t)gridDim.x * blockDim.x) {
-        const double a = packed_row(ent, __ldg(rp + r), __ldg(rp + r + 1), y, spal);
+    row_sums(R, OneVector{x}, spal, [&](int64_t r, const double (&s)[1]) { y[r] = s[0]; });
+}
+
+__global__ void __launch_bounds__(kSpmvThreads)
+    spmv_A2_kernel(SpmvRows R, const double *__restrict__ x, const double *__restrict__ c,
+                   const double *__restrict__ z, double *__restrict__ Ax, double *__restrict__ Acz, Palette pal) {
+    __shared__ double spal[16];
+    if (threadIdx.x < 16) spal[threadIdx.x] = pal.v[threadIdx.x];
+    __syncthreads();
+    row_sums(R, XAndCz{x, c, z}, spal, [&](int64_t r, const double (&s)[2]) {
+        Ax[r] = s[0];
+        Acz[r] = s[1];
+    });
+}
+
+__global__ void __launch_bounds__(kSpmvThreads)
+    spmv_AT_U_kernel(SpmvRows R, const double *__restrict__ y, const double *__restrict__ x,
+                     const double *__restrict__ c, double mu, double *__restrict__ ATy, double *__restrict__ U,
+                     Palette pal) {
+    __shared__ double spal[16];
+    if (threadIdx.x < 16) spal[threadIdx.x] = pal.v[threadIdx.x];
+    __syncthreads();
+    row_sums(R, OneVector{y}, spal, [&](int64_t r, const double (&s)[1]) {
+        const double a = s[0];
         ATy[r] = a;
         U[r] = mu * x[r] + a - c[r];
-    }
+    });
 }
 
 // ------------------------------------------------------------------ CG
@@ -640,15 +729,42 @@ __global__ void stats_kernel(const double *__restrict__ Ax, const double *__rest
     double s[4] = {0.0, 0.0, 0.0, 0.0};
     const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t j = gtid; j < nd; j += stride) {
-        const double d = Ax[j] - b[j];
-        s[0] += d * d;
-        s[3] += b[j] * y[j];
+    // kBatch elements' loads in flight; each sum keeps its order
+    constexpr int kBatch = 4;
+    for (int64_t j0 = gtid; j0 < nd; j0 += kBatch * stride) {
+        double va[kBatch], vb[kBatch], vy[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int64_t j = j0 + u * stride;
+            va[u] = j < nd ? Ax[j] : 0.0;
+            vb[u] = j < nd ? b[j] : 0.0;
+            vy[u] = j < nd ? y[j] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; u++)
+            if (j0 + u * stride < nd) {
+                const double d = va[u] - vb[u];
+                s[0] += d * d;
+                s[3] += vb[u] * vy[u];
+            }
     }
-    for (int64_t i = gtid; i < np; i += stride) {
-        const double d = ATy[i] + z[i] - c[i];
-        s[1] += d * d;
-        s[2] += c[i] * x[i];
+    for (int64_t i0 = gtid; i0 < np; i0 += kBatch * stride) {
+        double va[kBatch], vz[kBatch], vc[kBatch], vx[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int64_t i = i0 + u * stride;
+            va[u] = i < np ? ATy[i] : 0.0;
+            vz[u] = i < np ? z[i] : 0.0;
+            vc[u] = i < np ? c[i] : 0.0;
+            vx[u] = i < np ? x[i] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; u++)
+            if (i0 + u * stride < np) {
+                const double d = va[u] + vz[u] - vc[u];
+                s[1] += d * d;
+                s[2] += vc[u] * vx[u];
+            }
     }
     for (int k = 0; k < 4; k++) {
         const double v = block_sum(s[k], red);
@@ -687,8 +803,18 @@ __global__ void stats_kernel(const double *__restrict__ Ax, const double *__rest
 // middle factor of U+ = V P V^T,
 //     P_ii = max(t_ii, 0),   P_ij = t_ij (t_ii+ - t_jj+) / (t_ii - t_jj)   (i != j),
 // (with raw != 0: the rotated T itself, for callers that want eigenvalues)
-// and replays the recorded rotations on Vt (rows p, q of Vt per rotation),
-// leaving the refined eigenvectors for the next iteration.
+// and rotates Vt likewise (rows p, q of Vt per rotation), leaving the refined
+// eigenvectors for the next iteration: up to kJacobiFoldDim rows Vt lies in
+// shared memory beside T and takes each step's rotations with it; above, T's
+// rotations are recorded and replayed on Vt once T has made room for it.
+//
+// Bound by latency: a step is a chain of square roots and divisions, then two
+// barriers; a warp takes a pair row P, its lanes the columns, and skips the row
+// if nothing rotates it.  One nearly diagonal block of 10, 24, 64, 160 rows: 29,
+// 80, 363, 3,126 us; with a list of the rotated pairs made between two more
+// barriers, rows of even length and a replay for every block 40, 102, 573,
+// 5,817 us.  Fewer threads are no faster on small blocks (10 rows: 29 us with
+// 256, 35 with 128).
 __global__ void __launch_bounds__(kJacobiThreads)
     jacobi_warm_kernel(const double *__restrict__ T0, double *__restrict__ Pout,
                        double *__restrict__ Vt, const int64_t *__restrict__ boff,
@@ -702,13 +828,35 @@ __global__ void __launch_bounds__(kJacobiThreads)
     const int64_t off = boff[blk];
     const int np = n + (n & 1);
     const int m = np / 2;
-    double *T = sm;                                   // np*np (later: Vt)
-    double2 *cs = (double2 *)(T + (size_t)np * np);   // m
-    int *act = (int *)(cs + m);                       // m
-    int *alist = act + m;                             // m
+    const int ld = np + 1;
+    const bool fold = n <= kJacobiFoldDim;
+    double *T = sm;                      // np x ld
+    double *V = fold ? T + (size_t)np * ld : T;   // np x ld, rows = eigenvectors
+    double2 *cs = (double2 *)(V + (size_t)np * ld);   // m
+    int *act = (int *)(cs + m);          // m
     __shared__ double red[32];
-    __shared__ int nrot, nstep;
     __shared__ double s_nrm;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    double *Vb = Vt + off;
+    auto load_V = [&]() {
+        for (int i = warp; i < np; i += warps)
+            for (int j = lane; j < np; j += 32)
+                V[i * ld + j] = (i < n && j < n) ? Vb[(int64_t)i * n + j] : (i == j ? 1.0 : 0.0);
+    };
+    // rows p, q of V by the rotations of step st in cs, act
+    auto rotate_V = [&](int st) {
+        for (int P = warp; P < m; P += warps) {
+            if (!act[P]) continue;
+            const double2 r = cs[P];
+            int p, q;
+            rr_pair(st, P, np, p, q);
+            for (int j = lane; j < np; j += 32) {
+                const double vp = V[p * ld + j], vq = V[q * ld + j];
+                V[p * ld + j] = r.x * vp - r.y * vq;
+                V[q * ld + j] = r.y * vp + r.x * vq;
+            }
+        }
+    };
 
     const double *Tb = T0 + off;
     double fro = 0.0;
@@ -716,9 +864,10 @@ __global__ void __launch_bounds__(kJacobiThreads)
         const int i = e / np, j = e % np;
         double v = 0.0;
         if (i < n && j < n) v = 0.5 * (Tb[(int64_t)i * n + j] + Tb[(int64_t)j * n + i]);
-        T[e] = v;
+        T[i * ld + j] = v;
         fro += v * v;
     }
+    if (fold) load_V();
     fro = block_sum(fro, red);
     if (threadIdx.x == 0) s_nrm = sqrt(fro);
     __syncthreads();
@@ -726,64 +875,49 @@ __global__ void __launch_bounds__(kJacobiThreads)
     const double atol = abs_tol * nrm + 1e-300, gtol = gap_tol * nrm;
 
     double2 *rb = rot + rot_off[blk];
-    // per-step rotation counts live after the block's rotation record
-    int *scount = (int *)(rb + (int64_t)max_sweeps * (np - 1) * m);
-    int sweep = 0, total = 0;
+    int sweep = 0, total = 0, nrot = 0;   // the same on every thread
     for (; sweep < max_sweeps; sweep++) {
-        if (threadIdx.x == 0) nrot = 0;
-        __syncthreads();
+        nrot = 0;
         for (int st = 0; st < np - 1; st++) {
-            if (threadIdx.x == 0) nstep = 0;
-            __syncthreads();
-            for (int k = threadIdx.x; k < m; k += blockDim.x) {
+            const int k = threadIdx.x;   // blockDim.x >= m: a thread a pair
+            int a = 0;
+            if (k < m) {
                 int p, q;
                 rr_pair(st, k, np, p, q);
                 double c = 1.0, s = 0.0;
-                int a = 0;
                 if (q < n) {
-                    const double apq = T[p * np + q];
-                    const double app = T[p * np + p], aqq = T[q * np + q];
+                    const double apq = T[p * ld + q];
+                    const double app = T[p * ld + p], aqq = T[q * ld + q];
                     if (fabs(apq) > atol && apq * apq > gtol * fabs(aqq - app)) {
                         const double tau = (aqq - app) / (2.0 * apq);
-                        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + hypot(1.0, tau));
+                        // a correctly rounded reciprocal is 1.0 / x, in half the time
+                        const double r = __drcp_rn(fabs(tau) + hypot(1.0, tau)), t = tau >= 0.0 ? r : -r;
                         c = 1.0 / sqrt(1.0 + t * t);
                         s = t * c;
                         a = 1;
-                        atomicAdd(&nstep, 1);
                     }
                 }
                 cs[k] = make_double2(c, s);
                 act[k] = a;
-                rb[((int64_t)sweep * (np - 1) + st) * m + k] = make_double2(c, s);
+                if (!fold) rb[((int64_t)sweep * (np - 1) + st) * m + k] = make_double2(c, s);
             }
-            __syncthreads();
-            const int active = nstep;
-            if (threadIdx.x == 0) nrot += active;
-            if (active) {
-                // compact list of the rotated pairs of this step (warp 0, ballots)
-                if (threadIdx.x < 32) {
-                    const int lane = threadIdx.x;
-                    int base = 0;
-                    for (int k0 = 0; k0 < m; k0 += 32) {
-                        const int k = k0 + lane;
-                        const int a = (k < m) ? act[k] : 0;
-                        const unsigned bal = __ballot_sync(0xffffffffu, a);
-                        if (a) alist[base + __popc(bal & ((1u << lane) - 1u))] = k;
-                        base += __popc(bal);
-                    }
-                }
-                __syncthreads();
-                // 2x2 blocks (P, Q) with P rotated; a block with both P and Q
-                // rotated is handled once, by the smaller of the two
-                for (int it = threadIdx.x; it < active * m; it += blockDim.x) {
-                    const int P = alist[it / m], Q = it % m;
+            const int active = __syncthreads_count(a);
+            if (active == 0) continue;
+            nrot += active;
+            // 2x2 blocks (P, Q) with P rotated; a block with both P and Q
+            // rotated is handled once, by the smaller of the two
+            for (int P = warp; P < m; P += warps) {
+                if (!act[P]) continue;
+                const double2 cp = cs[P];
+                int pP, qP;
+                rr_pair(st, P, np, pP, qP);
+                for (int Q = lane; Q < m; Q += 32) {
                     if (act[Q] && Q < P) continue;
-                    const double2 cp = cs[P], cq = cs[Q];
-                    int pP, qP, pQ, qQ;
-                    rr_pair(st, P, np, pP, qP);
+                    const double2 cq = cs[Q];
+                    int pQ, qQ;
                     rr_pair(st, Q, np, pQ, qQ);
-                    const double b11 = T[pP * np + pQ], b12 = T[pP * np + qQ];
-                    const double b21 = T[qP * np + pQ], b22 = T[qP * np + qQ];
+                    const double b11 = T[pP * ld + pQ], b12 = T[pP * ld + qQ];
+                    const double b21 = T[qP * ld + pQ], b22 = T[qP * ld + qQ];
                     const double m11 = b11 * cq.x - b12 * cq.y, m12 = b11 * cq.y + b12 * cq.x;
                     const double m21 = b21 * cq.x - b22 * cq.y, m22 = b21 * cq.y + b22 * cq.x;
                     double n11 = cp.x * m11 - cp.y * m21, n12 = cp.x * m12 - cp.y * m22;
@@ -791,25 +925,23 @@ __global__ void __launch_bounds__(kJacobiThreads)
                     if (P == Q) {
                         n12 = 0.0;
                         n21 = 0.0;
-                        T[pP * np + pP] = n11;
-                        T[pP * np + qP] = n12;
-                        T[qP * np + pP] = n21;
-                        T[qP * np + qP] = n22;
+                        T[pP * ld + pP] = n11;
+                        T[pP * ld + qP] = n12;
+                        T[qP * ld + pP] = n21;
+                        T[qP * ld + qP] = n22;
                     } else {
-                        T[pP * np + pQ] = n11; T[pQ * np + pP] = n11;
-                        T[pP * np + qQ] = n12; T[qQ * np + pP] = n12;
-                        T[qP * np + pQ] = n21; T[pQ * np + qP] = n21;
-                        T[qP * np + qQ] = n22; T[qQ * np + qP] = n22;
+                        T[pP * ld + pQ] = n11; T[pQ * ld + pP] = n11;
+                        T[pP * ld + qQ] = n12; T[qQ * ld + pP] = n12;
+                        T[qP * ld + pQ] = n21; T[pQ * ld + qP] = n21;
+                        T[qP * ld + qQ] = n22; T[qQ * ld + qP] = n22;
                     }
                 }
             }
-            if (threadIdx.x == 0) scount[(int64_t)sweep * (np - 1) + st] = active;
+            if (fold) rotate_V(st);
             __syncthreads();
         }
         total += nrot;
-        const int done = (nrot == 0);
-        __syncthreads();
-        if (done) {
+        if (nrot == 0) {
             sweep++;
             break;
         }
@@ -823,63 +955,41 @@ __global__ void __launch_bounds__(kJacobiThreads)
     double *Pb = Pout + off;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int i = e / n, j = e % n;
-        const double li = T[i * np + i];
+        const double li = T[i * ld + i];
         double pv;
         if (raw) {
-            pv = T[i * np + j];   // the rotated matrix itself (its diagonal: the eigenvalues)
+            pv = T[i * ld + j];   // the rotated matrix itself (its diagonal: the eigenvalues)
         } else if (i == j) {
             pv = fmax(li, 0.0);
         } else {
-            const double lj = T[j * np + j];
+            const double lj = T[j * ld + j];
             const double pi = fmax(li, 0.0), pj = fmax(lj, 0.0);
             const double gam = (li != lj) ? (pi - pj) / (li - lj) : (li > 0.0 ? 1.0 : 0.0);
-            pv = gam * T[i * np + j];
+            pv = gam * T[i * ld + j];
         }
         Pb[e] = pv;
     }
     __syncthreads();
 
-    // replay the rotations on Vt (rows = eigenvectors)
-    double *V = T;
-    double *Vb = Vt + off;
-    for (int e = threadIdx.x; e < np * np; e += blockDim.x) {
-        const int i = e / np, j = e % np;
-        V[e] = (i < n && j < n) ? Vb[(int64_t)i * n + j] : (i == j ? 1.0 : 0.0);
-    }
-    __syncthreads();
-    for (int sw = 0; sw < sweep; sw++) {
-        for (int st = 0; st < np - 1; st++) {
-            if (scount[(int64_t)sw * (np - 1) + st] == 0) continue;   // uniform across the CTA
-            const double2 *rs = rb + ((int64_t)sw * (np - 1) + st) * m;
-            if (threadIdx.x < 32) {
-                const int lane = threadIdx.x;
-                int base = 0;
-                for (int k0 = 0; k0 < m; k0 += 32) {
-                    const int k = k0 + lane;
-                    const int a = (k < m) ? (rs[k].y != 0.0) : 0;
-                    const unsigned bal = __ballot_sync(0xffffffffu, a);
-                    if (a) alist[base + __popc(bal & ((1u << lane) - 1u))] = k;
-                    base += __popc(bal);
-                }
-                if (lane == 0) nstep = base;
+    if (!fold) {
+        // replay the rotations on Vt; a step's are fetched during the one before
+        load_V();
+        const int steps = sweep * (np - 1), k = threadIdx.x;
+        double2 r = k < m && steps > 0 ? rb[k] : make_double2(1.0, 0.0);
+        for (int q = 0, st = 0; q < steps; q++, st = st + 1 == np - 1 ? 0 : st + 1) {
+            if (k < m) {
+                cs[k] = r;
+                act[k] = r.y != 0.0;
             }
-            __syncthreads();
-            const int active = nstep;
-            for (int it = threadIdx.x; it < active * np; it += blockDim.x) {
-                const int k = alist[it / np], j = it % np;
-                const double2 r = rs[k];
-                int p, q;
-                rr_pair(st, k, np, p, q);
-                const double vp = V[p * np + j], vq = V[q * np + j];
-                V[p * np + j] = r.x * vp - r.y * vq;
-                V[q * np + j] = r.y * vp + r.x * vq;
-            }
+            const int active = __syncthreads_count(r.y != 0.0);
+            if (k < m && q + 1 < steps) r = rb[(int64_t)(q + 1) * m + k];
+            if (active) rotate_V(st);
             __syncthreads();
         }
     }
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int i = e / n, j = e % n;
-        Vb[e] = V[i * np + j];
+        Vb[e] = V[i * ld + j];
     }
 }
 

@@ -18,6 +18,7 @@ struct CgRows {
 };
 constexpr int kJacobiThreads = 512;
 constexpr int kJacobiMaxDim = 160;     // np*np doubles + rotations must fit in 227 KB
+constexpr int kJacobiFoldDim = 80;     // up to here V is rotated beside T: 2 CTAs still fit an SM
 constexpr int kStatsBlocks = 256;
 
 struct Palette {
@@ -60,18 +61,21 @@ __host__ __device__ inline uint32_t cg_table_words(uint32_t nslices, uint32_t ne
 }
 constexpr size_t kCgStaticSmem = 4096;   // at least the kernel's static shared memory
 
-__global__ void spmv_kernel(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ent,
-                            int64_t nrows, const double *__restrict__ x, double *__restrict__ y,
-                            Palette pal);
-__global__ void spmv_A2_kernel(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ent,
-                               int64_t nrows, const double *__restrict__ x,
-                               const double *__restrict__ c, const double *__restrict__ z,
-                               double *__restrict__ Ax, double *__restrict__ Acz, Palette pal);
-__global__ void spmv_AT_U_kernel(const uint32_t *__restrict__ rp,
-                                 const uint32_t *__restrict__ ent, int64_t nrows,
-                                 const double *__restrict__ y, const double *__restrict__ x,
-                                 const double *__restrict__ c, double mu,
-                                 double *__restrict__ ATy, double *__restrict__ U, Palette pal);
+// Packed rows of A or A^T (CSR) and the list of those longer than
+// kSpmvLongRow, which the first long_blocks CTAs take
+constexpr uint32_t kSpmvLongRow = 32;
+struct SpmvRows {
+    const uint32_t *rp, *ent, *long_rows;
+    int64_t nrows;
+    uint32_t nlong, long_blocks;
+};
+__global__ void spmv_kernel(SpmvRows R, const double *__restrict__ x, double *__restrict__ y, Palette pal);
+__global__ void spmv_A2_kernel(SpmvRows R, const double *__restrict__ x, const double *__restrict__ c,
+                               const double *__restrict__ z, double *__restrict__ Ax, double *__restrict__ Acz,
+                               Palette pal);
+__global__ void spmv_AT_U_kernel(SpmvRows R, const double *__restrict__ y, const double *__restrict__ x,
+                                 const double *__restrict__ c, double mu, double *__restrict__ ATy,
+                                 double *__restrict__ U, Palette pal);
 // the CG starting point of the next outer iteration from the last dual
 // solutions (order 0: y itself, 1: 2y - y1, 2: 3y - 3y1 + y2); y1, y2 shift
 __global__ void extrapolate_y_kernel(double *__restrict__ y, double *__restrict__ y1,
@@ -104,7 +108,12 @@ unsigned long long current_context_id();
 
 inline size_t jacobi_smem_bytes(int n) {
     const int np = n + (n & 1);
-    return (size_t)np * np * sizeof(double) + (size_t)(np / 2) * (sizeof(double2) + 2 * sizeof(int));
+    // T with odd rows (columns free of bank conflicts); V beside it up to
+    // kJacobiFoldDim rows; monotone in n, so that the largest block's size serves all
+    const size_t one = (size_t)np * (np + 1) * sizeof(double);
+    constexpr size_t fold = 2 * (size_t)kJacobiFoldDim * (kJacobiFoldDim + 1) * sizeof(double);
+    const size_t mats = n <= kJacobiFoldDim ? 2 * one : (one > fold ? one : fold);
+    return mats + (size_t)(np / 2) * (sizeof(double2) + sizeof(int));
 }
 
 }  // namespace v2b

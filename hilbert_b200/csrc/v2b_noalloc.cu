@@ -38,9 +38,8 @@ constexpr int kNoAllocMaxDim = 128;
 constexpr int kNoAllocSweeps = 30;   // the library projection's Jacobi sweep limit
 constexpr int kNoAllocPairs = kNoAllocMaxDim / 2;
 constexpr int64_t kNoAllocMat = (int64_t)kNoAllocMaxDim * kNoAllocMaxDim;   // doubles per matrix
-// rotation record + per-step counts (in double2 units), as jacobi_warm_kernel lays them out
-constexpr int64_t kNoAllocRot = (int64_t)kNoAllocSweeps * (kNoAllocMaxDim - 1) * kNoAllocPairs +
-                                ((int64_t)kNoAllocSweeps * (kNoAllocMaxDim - 1) + 3) / 4 + 1;
+// rotation record, as jacobi_warm_kernel lays it out
+constexpr int64_t kNoAllocRot = (int64_t)kNoAllocSweeps * (kNoAllocMaxDim - 1) * kNoAllocPairs;
 constexpr int kNoAllocTiles = (kNoAllocMaxDim / kGemmTile) * (kNoAllocMaxDim / kGemmTile);
 
 // layout of the scratch array, in 256-byte aligned sections

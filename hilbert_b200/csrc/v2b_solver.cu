@@ -107,8 +107,9 @@ int sm_count() {
 }
 
 struct DeviceOp {
-    uint32_t *rp = nullptr, *ent = nullptr;
+    uint32_t *rp = nullptr, *ent = nullptr, *long_rows = nullptr;
     int64_t nrows = 0;
+    uint32_t nlong = 0;
     size_t nnz = 0;
     v2b::Palette pal{};
 
@@ -120,10 +121,25 @@ struct DeviceOp {
         V2B_CK(cudaMemcpy(rp, op.row_ptr.data(), op.row_ptr.size() * 4, cudaMemcpyHostToDevice));
         V2B_CK(cudaMemcpy(ent, op.entries.data(), nnz * 4, cudaMemcpyHostToDevice));
         for (int i = 0; i < 16; i++) pal.v[i] = i < (int)op.palette.size() ? op.palette[i] : 0.0;
+        std::vector<uint32_t> lr;
+        for (int64_t r = 0; r < nrows; r++)
+            if (op.row_ptr[r + 1] - op.row_ptr[r] > v2b::kSpmvLongRow) lr.push_back((uint32_t)r);
+        nlong = (uint32_t)lr.size();
+        long_rows = dalloc<uint32_t>(lr.size());
+        if (nlong) V2B_CK(cudaMemcpy(long_rows, lr.data(), lr.size() * 4, cudaMemcpyHostToDevice));
+    }
+    // the rows as the map kernels take them, and their grid
+    v2b::SpmvRows rows() const {
+        constexpr uint32_t warps = v2b::kSpmvThreads / 32;
+        return v2b::SpmvRows{rp, ent, long_rows, nrows, nlong, (nlong + warps - 1) / warps};
+    }
+    int grid() const {
+        const int64_t g = (nrows + v2b::kSpmvThreads - 1) / v2b::kSpmvThreads;
+        return (int)rows().long_blocks + (int)std::max<int64_t>(1, std::min<int64_t>(g, 148 * 16));
     }
     void release() {
-        for (void *p : {(void *)rp, (void *)ent}) cudaFree(p);
-        rp = ent = nullptr;
+        for (void *p : {(void *)rp, (void *)ent, (void *)long_rows}) cudaFree(p);
+        rp = ent = long_rows = nullptr;
     }
 };
 
@@ -528,9 +544,8 @@ struct ProjectPlan {
                 const int np = d[i] + (d[i] & 1);
                 h_roff_small[i] = ro;
                 nsmall++;
-                // rotation record (max_sweeps x steps x pairs) + per-step counts
-                ro += (int64_t)max_sweeps * std::max(np - 1, 0) * (np / 2) +
-                      ((int64_t)max_sweeps * std::max(np - 1, 0) + 3) / 4 + 1;
+                // rotation record (max_sweeps x steps x pairs), where one is kept
+                if (d[i] > v2b::kJacobiFoldDim) ro += (int64_t)max_sweeps * (np - 1) * (np / 2);
                 smem = std::max(smem, v2b::jacobi_smem_bytes(d[i]));
             } else {
                 h_roff_big[i] = rb;
@@ -922,7 +937,7 @@ struct ProjectPlan {
             croff.push_back(roff);
             if (kind == 1) {
                 const int np = j.k + (j.k & 1);
-                roff += (int64_t)max_sweeps * (np - 1) * (np / 2) + ((int64_t)max_sweeps * (np - 1) + 3) / 4 + 1;
+                if (j.k > kJacobiFoldDim) roff += (int64_t)max_sweeps * (np - 1) * (np / 2);
                 nmid++;
             } else {
                 roff += big_record_slots(j.k, kBigSweeps);
@@ -1499,14 +1514,12 @@ struct v2b_problem {
     }
 
     void Au(const double *in, double *out, cudaStream_t s) {
-        v2b::spmv_kernel<<<grid_for(A.nrows, v2b::kSpmvThreads), v2b::kSpmvThreads, 0, s>>>(
-            A.rp, A.ent, A.nrows, in, out, A.pal);
+        v2b::spmv_kernel<<<A.grid(), v2b::kSpmvThreads, 0, s>>>(A.rows(), in, out, A.pal);
         V2B_CK(cudaGetLastError());
         launches++;
     }
     void ATu(const double *in, double *out, cudaStream_t s) {
-        v2b::spmv_kernel<<<grid_for(AT.nrows, v2b::kSpmvThreads), v2b::kSpmvThreads, 0, s>>>(
-            AT.rp, AT.ent, AT.nrows, in, out, AT.pal);
+        v2b::spmv_kernel<<<AT.grid(), v2b::kSpmvThreads, 0, s>>>(AT.rows(), in, out, AT.pal);
         V2B_CK(cudaGetLastError());
         launches++;
     }
@@ -1540,8 +1553,7 @@ struct v2b_problem {
         launch_cg(o.cg_convergence, o.cg_maxiter);
         mark(0, 1);
         mark(1, 0);
-        v2b::spmv_AT_U_kernel<<<grid_for(np, v2b::kSpmvThreads), v2b::kSpmvThreads, 0, stream>>>(
-            AT.rp, AT.ent, np, y, x, c, mu, ATy, U, AT.pal);
+        v2b::spmv_AT_U_kernel<<<AT.grid(), v2b::kSpmvThreads, 0, stream>>>(AT.rows(), y, x, c, mu, ATy, U, AT.pal);
         V2B_CK(cudaGetLastError());
         launches++;
         mark(1, 1);
@@ -1550,8 +1562,7 @@ struct v2b_problem {
         plan.project(U, mu, x, z, stream, launches);
         mark(2, 1);
         mark(3, 0);
-        v2b::spmv_A2_kernel<<<grid_for(nd, v2b::kSpmvThreads), v2b::kSpmvThreads, 0, stream>>>(
-            A.rp, A.ent, nd, x, c, z, Ax, Acz, A.pal);
+        v2b::spmv_A2_kernel<<<A.grid(), v2b::kSpmvThreads, 0, stream>>>(A.rows(), x, c, z, Ax, Acz, A.pal);
         V2B_CK(cudaGetLastError());
         launches++;
         mark(3, 1);
@@ -1631,8 +1642,7 @@ struct v2b_problem {
             V2B_CK(cudaMemsetAsync(z, 0, np * 8, stream));
         }
         V2B_CK(cudaMemsetAsync(status, 0, 8, stream));
-        v2b::spmv_A2_kernel<<<grid_for(nd, v2b::kSpmvThreads), v2b::kSpmvThreads, 0, stream>>>(
-            A.rp, A.ent, nd, x, c, z, Ax, Acz, A.pal);
+        v2b::spmv_A2_kernel<<<A.grid(), v2b::kSpmvThreads, 0, stream>>>(A.rows(), x, c, z, Ax, Acz, A.pal);
         V2B_CK(cudaGetLastError());
         launches++;
         long oiter = 0, iiter = 0;

@@ -1,0 +1,49 @@
+"""The map kernels' split of rows (a thread for a short one, a warp with chunks
+of 128 entries for a long one) and the one-CTA Jacobi kernel around its edges."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import hilbert_b200 as hb
+from hilbert_b200 import _capi
+from oracle.bpsdp import project_blocks
+from oracle.maps import OracleProblem
+
+pytestmark = pytest.mark.gpu
+
+
+# rows of up to n^2 entries: 1 to 36, 121 (one chunk), 169 (two)
+@pytest.mark.parametrize("n,na,nb,pos", [(1, 1, 1, "DQG"), (5, 3, 2, "DQG"), (6, 3, 3, "DQGT1T2"),
+                                         (11, 6, 6, "DQG"), (13, 7, 6, "DG")])
+def test_rows_bit_exact(cuda_device, n, na, nb, pos):
+    import torch
+    rng = np.random.default_rng(n)
+    o = OracleProblem(n, na, nb, pos, 1, 1, h=rng.standard_normal((n, n)), g=rng.standard_normal((n,) * 4))
+    p = hb.V2RDMProblem(n, na, nb, pos)
+    x, y = rng.standard_normal(o.n_primal), rng.standard_normal(o.n_dual)
+    assert np.array_equal(p.Au(torch.from_numpy(x).to(cuda_device)).cpu().numpy(), o.Au(x))
+    assert np.array_equal(p.ATu(torch.from_numpy(y).to(cuda_device)).cpu().numpy(), o.ATu(y))
+    p.close()
+
+
+# odd sizes, one warp of pairs and more, both sides of the size up to which the
+# eigenvectors stay in shared memory
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 33, 63, 66, 79, 80, 81, 82, 127, 128])
+@pytest.mark.parametrize("spec", ["normal", "zero"])
+def test_one_cta_jacobi(cuda_device, n, spec):
+    import torch
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n))
+    U = {"normal": a + a.T, "zero": 0.0 * a}[spec].ravel()
+    xr, zr = project_blocks(U, [n], 0.5)
+    d = torch.from_numpy(U).to(cuda_device)
+    x, z = torch.full_like(d, float("nan")), torch.full_like(d, float("nan"))
+    rc = _capi.load().v2b_project_block_noalloc(
+        ctypes.c_void_p(d.data_ptr()), n, 0.5, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(z.data_ptr()),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == _capi.V2B_OK
+    # 10 sweeps of n rotations a row, each rounding by a few eps: 10 * 128 * 4 eps
+    tol = 1.2e-12 * max(np.linalg.norm(U), 1e-300)
+    assert np.max(np.abs(x.cpu().numpy() - xr)) <= 2 * tol   # x = U+ / mu
+    assert np.max(np.abs(z.cpu().numpy() - zr)) <= tol

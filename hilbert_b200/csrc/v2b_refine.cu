@@ -44,15 +44,15 @@ __device__ __forceinline__ double gamma_pq(double li, double lj) {
     return (li != lj) ? (pi - pj) / (li - lj) : (li > 0.0 ? 1.0 : 0.0);
 }
 
-// Row pairs (r, n-1-r) hold n-1 upper-triangle pairs together: CTA s of a
-// block takes row pairs [s R, (s+1) R), R = ceil(ceil(n/2) / kClassifySplit).
+// CTA s of a block takes the row pairs (r, n-1-r), r in [s R, (s+1) R),
+// R = ceil(ceil(n/2) / kNormSplit).
 __device__ __forceinline__ void split_rows(int n, int s, int &r0, int &r1) {
-    const int half = (n + 1) / 2, R = (half + kClassifySplit - 1) / kClassifySplit;
+    const int half = (n + 1) / 2, R = (half + kNormSplit - 1) / kNormSplit;
     r0 = min(half, s * R);
     r1 = min(half, (s + 1) * R);
 }
 
-// Frobenius norms of the symmetrised blocks, in kClassifySplit partial sums per
+// Frobenius norms of the symmetrised blocks, in kNormSplit partial sums per
 // block (summed in a fixed order by the readers: the result is deterministic)
 __global__ void __launch_bounds__(256)
     block_norm_kernel(const double *__restrict__ Us, const int64_t *__restrict__ boff,
@@ -63,28 +63,42 @@ __global__ void __launch_bounds__(256)
     split_rows(n, sidx, r0, r1);
     const double *Ub = Us + boff[blk];
     double acc = 0.0;
-    for (int r = r0; r < r1; r++)
-        for (int side = 0; side < 2; side++) {
-            const int row = side ? n - 1 - r : r;
-            if (side && row == r) continue;   // the middle row of an odd block
-            for (int c = threadIdx.x; c < n; c += blockDim.x) {
-                const double v = Ub[(int64_t)row * n + c];
-                acc += v * v;
-            }
+    // the CTA's rows r0, n-1-r0, r0+1, ..., each in strides of the CTA; added
+    // one by one, kBatch loads in flight
+    constexpr int kBatch = 8;
+    const int tid = threadIdx.x, rows = 2 * (r1 - r0) - (2 * r1 > n ? 1 : 0);   // the middle row once
+    int u = 0, c = tid;
+    while (u < rows && c < n) {
+        double v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) {
+            const bool in = u < rows;   // else a load of no use, so that none waits for a branch
+            const int r = r0 + (u >> 1), row = (u & 1) ? n - 1 - r : r;
+            const double w = Ub[in ? (int64_t)row * n + c : 0];
+            v[k] = in ? w : 0.0;
+            const int next = c + (int)blockDim.x;
+            u += next >= n;
+            c = next >= n ? tid : next;
         }
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) acc += v[k] * v[k];
+    }
     acc = block_sum(acc, red);
-    if (threadIdx.x == 0) part[blk * kClassifySplit + sidx] = acc;
+    if (threadIdx.x == 0) part[blk * kNormSplit + sidx] = acc;
 }
 
 __device__ __forceinline__ double block_norm(const double *part, int blk) {
     double s = 0.0;
-    for (int k = 0; k < kClassifySplit; k++) s += part[blk * kClassifySplit + k];
+    for (int k = 0; k < kNormSplit; k++) s += part[blk * kNormSplit + k];
     return sqrt(s);
 }
 
-// Acceptance test, kClassifySplit CTAs per block.  Failing pairs are counted
-// and non-separable ones recorded as edges; the last CTA of a block to finish
-// sets its state (done -> done_stamp = stamp, for write_p_kernel).
+// Acceptance test, gridDim.y CTAs per block: the pairs of 32 x 32 tiles (I, J),
+// (J, I), read along rows and turned in shared memory.  Failing pairs are
+// counted and non-separable ones recorded as edges; the last CTA of a block to
+// finish sets its state (done -> done_stamp = stamp, for write_p_kernel).
+// (20e,20o), all blocks: 24 us; with columns read from memory by 16 CTAs a
+// block 72.
 __global__ void __launch_bounds__(kRefineThreads)
     refine_classify_kernel(const double *__restrict__ T, const int64_t *__restrict__ boff,
                            const int *__restrict__ bdim, int *__restrict__ bstate,
@@ -99,28 +113,36 @@ __global__ void __launch_bounds__(kRefineThreads)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
     int *cnt = counts + 3 * blk;   // [0] failing pairs, [1] edges, [2] finished CTAs
     __shared__ int s_last;
-    extern __shared__ double dg[];   // n diagonal entries
+    __shared__ double up[32][33], lo[32][33], dg[2][32];   // T[I, J], T[J, I], their diagonals
     const int64_t off = boff[blk];
     const double *Tb = T + off;
     const double nrm = block_norm(part, blk);
     const double atol = abs_tol * nrm, gtol = gap_tol * nrm;
-    for (int i = tid; i < n; i += blockDim.x) dg[i] = Tb[(int64_t)i * n + i];
-    __syncthreads();
-    int r0, r1;
-    split_rows(n, sidx, r0, r1);
     int bad = 0;
     int2 *eb = h_edges + (int64_t)blk * kRefineEdgeCap;
-    // rows r0..r1-1 and their partners n-1-r, one warp per row
-    for (int w = warp; w < 2 * (r1 - r0); w += nwarp) {
-        const int r = r0 + (w >> 1);
-        const int i = (w & 1) ? n - 1 - r : r;
-        if ((w & 1) && i == r) continue;
-        const double di = dg[i];
-        for (int j = i + 1 + lane; j < n; j += 32) {
-            const double t = 0.5 * (Tb[(int64_t)i * n + j] + Tb[(int64_t)j * n + i]);
+    const int nt = (n + 31) / 32, npairs = nt * (nt + 1) / 2;
+    for (int t = sidx; t < npairs; t += gridDim.y) {
+        int I = 0, J = t;
+        while (J >= nt - I) J -= nt - I++;
+        J += I;
+        const int i0 = 32 * I, j0 = 32 * J;
+        __syncthreads();
+        for (int r = warp; r < 32; r += nwarp) {
+            up[r][lane] = i0 + r < n && j0 + lane < n ? Tb[(int64_t)(i0 + r) * n + j0 + lane] : 0.0;
+            lo[r][lane] = j0 + r < n && i0 + lane < n ? Tb[(int64_t)(j0 + r) * n + i0 + lane] : 0.0;
+        }
+        if (warp < 2) {
+            const int i = (warp ? j0 : i0) + lane;
+            dg[warp][lane] = i < n ? Tb[(int64_t)i * n + i] : 0.0;
+        }
+        __syncthreads();
+        for (int r = warp; r < 32; r += nwarp) {
+            const int i = i0 + r, j = j0 + lane;
+            if (j <= i || j >= n) continue;   // i < j < n
+            const double t = 0.5 * (up[r][lane] + lo[lane][r]);
             const double at = fabs(t);
             if (at <= atol) continue;
-            const double dj = dg[j];
+            const double di = dg[0][r], dj = dg[1][lane];
             const double g = fabs(di - dj);
             const bool cross = (di >= 0.0) != (dj >= 0.0);
             const double delta = cross ? g : fmin(fabs(di), fabs(dj));
@@ -133,11 +155,12 @@ __global__ void __launch_bounds__(kRefineThreads)
             }
         }
     }
+    __syncwarp();
     bad = __reduce_add_sync(0xffffffffu, bad);
     if (lane == 0 && bad) atomicAdd(cnt, bad);
     __threadfence();
     __syncthreads();
-    if (tid == 0) s_last = (atomicAdd(cnt + 2, 1) == kClassifySplit - 1);
+    if (tid == 0) s_last = (atomicAdd(cnt + 2, 1) == (int)gridDim.y - 1);
     __syncthreads();
     if (!s_last) return;
     if (tid == 0) {

@@ -36,12 +36,17 @@ struct ClusterJob {
     int blk, k, moff, qoff;
 };
 
-constexpr int kClassifySplit = 16;   // CTAs per block in the acceptance test
+// CTAs per block in the acceptance test: two tile pairs each, up to 64 CTAs
+inline int classify_split(int max_dim) {
+    const int nt = (max_dim + 31) / 32, pairs = nt * (nt + 1) / 2;
+    return pairs < 128 ? (pairs + 1) / 2 : 64;
+}
+constexpr int kNormSplit = 16;   // CTAs per block in block_norm_kernel
 
-// Frobenius norms of the symmetrised blocks as kClassifySplit partial sums each
+// Frobenius norms of the symmetrised blocks as kNormSplit partial sums each
 __global__ void block_norm_kernel(const double *__restrict__ Us, const int64_t *__restrict__ boff,
                                   const int *__restrict__ bdim, double *__restrict__ part);
-// acceptance test and pair classification (grid nblk x kClassifySplit)
+// acceptance test and pair classification (grid nblk x classify_split)
 __global__ void refine_classify_kernel(const double *__restrict__ T, const int64_t *__restrict__ boff,
                                        const int *__restrict__ bdim, int *__restrict__ bstate,
                                        const unsigned long long *__restrict__ orth,

@@ -312,7 +312,7 @@ struct ProjectPlan {
     int *bstate = nullptr, *h_bstate_up = nullptr;   // device / pinned staging
     unsigned long long *orth = nullptr;
     double *bnorm = nullptr;
-    double *norm_part = nullptr;     // kClassifySplit partial squared norms per block
+    double *norm_part = nullptr;     // kNormSplit partial squared norms per block
     int *cls_counts = nullptr;       // per block: failing pairs, edges, finished CTAs
     int *done_stamp = nullptr;       // classify launch that accepted the block
     int stamp = 0;
@@ -341,11 +341,11 @@ struct ProjectPlan {
         int njobs = 0, ntiles = 0, kmax = 0;
     };
     std::vector<BJStep> bj_steps;
+    int classify_ctas = 1;        // CTAs per block in the acceptance test
     std::vector<int> bj_nsteps;   // steps per sweep of each block (0: not scheduled)
     unsigned char *bj_dev = nullptr;
     int *bj_on = nullptr, *h_bjon = nullptr;
     long refine_bj_sweeps = 0;
-    size_t classify_smem = 0;
     // recorded after a call's last upload from the pinned staging buffers; the
     // next call waits for it before writing them again
     cudaEvent_t staged = nullptr;
@@ -561,6 +561,7 @@ struct ProjectPlan {
         std::stable_sort(tl.begin(), tl.end(), [&](const int4 &a, const int4 &b) { return d[a.x] > d[b.x]; });
         ntiles = (int)tl.size();
         sms = sm_count();
+        classify_ctas = v2b::classify_split(maxn);
         gtile = maxn < kSplitMinDim && ntiles <= sms ? 32 : v2b::kGemmTile;
         std::vector<int4> gtl = tl;
         if (gtile == 32) {
@@ -614,7 +615,7 @@ struct ProjectPlan {
         bstate = dalloc<int>(nblk);
         orth = dalloc<unsigned long long>(nblk);
         bnorm = dalloc<double>(nblk);
-        norm_part = dalloc<double>((size_t)nblk * v2b::kClassifySplit);
+        norm_part = dalloc<double>((size_t)nblk * v2b::kNormSplit);
         cls_counts = dalloc<int>(3 * (size_t)nblk);
         done_stamp = dalloc<int>(nblk);
         V2B_CK(cudaMemset(cls_counts, 0, 3 * sizeof(int) * nblk));
@@ -637,9 +638,6 @@ struct ProjectPlan {
         Tc = dalloc<double>(total);
         Pc = dalloc<double>(total);
         V2B_CK(cudaMemcpy(rowbase, rb_host.data(), nblk * 4, cudaMemcpyHostToDevice));
-        classify_smem = (size_t)maxn * sizeof(double);
-        if (classify_smem > 48 * 1024)
-            V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::refine_classify_kernel, (int)classify_smem));
         V2B_CK(v2b::prepare_cluster_eig());
         V2B_CK(v2b::raise_dynamic_smem((const void *)v2b::bj_apply_kernel, v2b::kBjApplySmem));
         // clusters of kRefineSmallCluster+1 .. kJacobiMaxDim rows use jacobi_warm_kernel
@@ -1046,7 +1044,7 @@ struct ProjectPlan {
         V2B_CK(cudaMemcpyAsync(Tsave, T, total * sizeof(double), cudaMemcpyDeviceToDevice, s));
         // ||T||_F = ||sym(U)||_F for an orthonormal Vt: the tests use the block norms of Us
         ph_begin(1, s);
-        block_norm_kernel<<<dim3(nblk, kClassifySplit), 256, 0, s>>>(Us, boff, bdim, norm_part);
+        block_norm_kernel<<<dim3(nblk, kNormSplit), 256, 0, s>>>(Us, boff, bdim, norm_part);
         ph_end(s);
         V2B_CK(cudaGetLastError());
         launches++;
@@ -1088,7 +1086,7 @@ struct ProjectPlan {
             }
             ++stamp;
             ph_begin(1, s);
-            refine_classify_kernel<<<dim3(nblk, kClassifySplit), kRefineThreads, classify_smem, s>>>(
+            refine_classify_kernel<<<dim3(nblk, classify_ctas), kRefineThreads, 0, s>>>(
                 T, boff, bdim, bstate, orth, norm_part, gap_tol, abs_tol, bnorm, cls_counts, done_stamp,
                 stamp, d_state, d_nbad, d_nedge, d_edges);
             write_p_kernel<<<ntiles, 256, 0, s>>>(T, P, tiles, boff, bdim, done_stamp, stamp);

@@ -47,3 +47,25 @@ def test_one_cta_jacobi(cuda_device, n, spec):
     tol = 1.2e-12 * max(np.linalg.norm(U), 1e-300)
     assert np.max(np.abs(x.cpu().numpy() - xr)) <= 2 * tol   # x = U+ / mu
     assert np.max(np.abs(z.cpu().numpy() - zr)) <= tol
+
+
+# the acceptance test's 32-row tile pairs: blocks of one partial tile, of whole
+# tiles (64, 128), of a last tile of one to four rows (36, 66, 100), of seven
+@pytest.mark.parametrize("n,na,nb", [(5, 3, 2), (8, 4, 4), (9, 5, 4), (10, 5, 5)])
+@pytest.mark.parametrize("step", [1e-12, 1e-5, 1e-2])
+def test_acceptance_on_ragged_tiles(cuda_device, n, na, nb, step):
+    import torch
+    p = hb.V2RDMProblem(n, na, nb)
+    rng = np.random.default_rng(n)
+    def symmetric():
+        blocks = [rng.standard_normal((int(d), int(d))) for d in p.dims]
+        return np.concatenate([(a + a.T).ravel() for a in blocks])
+    U = symmetric()
+    for k in range(3):   # from scratch, then warm: accepted, rotated, restarted
+        V = U + k * step * symmetric()
+        xr, zr = project_blocks(V, p.dims, 0.8)
+        x, z = p.project(torch.from_numpy(V).to(cuda_device), 0.8, warm=True)
+        tol = 1e-11 * np.linalg.norm(V)   # as the other projection tests, which the acceptance rule sets
+        assert np.max(np.abs(x.cpu().numpy() - xr)) <= tol
+        assert np.max(np.abs(z.cpu().numpy() - zr)) <= tol
+    p.close()

@@ -88,12 +88,12 @@ def fp64_reference(workload):
 # available as a fixture.
 DEVICE_COUNTS = {"df20": {"outer_iterations": 4101, "cg_iterations": 127159}}
 # DRAM bytes the CG kernel moves per CG iteration (dram__bytes_read.sum +
-# dram__bytes_write.sum from one ncu capture of a whole launch: 9.56 + 4.70 GB
+# dram__bytes_write.sum from one ncu capture of a whole launch: 3.60 + 1.86 GB
 # over 142 iterations and the initial residual, on the same df20 problem;
 # `python -m hilbert_b200.synthetic --n 20 --naux 400 --max-outer 1`).  The
 # bench's launches run the same passes over the same vectors, so their traffic
 # is this figure times their iterations.
-CG_DRAM_BYTES_PER_ITERATION = {"df20": 14.26e9 / 143}
+CG_DRAM_BYTES_PER_ITERATION = {"df20": 5.46e9 / 143}
 
 
 def iteration_counts(workload):

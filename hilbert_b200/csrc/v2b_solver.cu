@@ -73,6 +73,12 @@ T *dalloc(size_t n) {
     return (T *)p;
 }
 
+// cudaMemcpy from pageable memory and cudaMemset may return before the device
+// holds their result, and the library's streams (non-blocking, as the caller's
+// may be) are not ordered with the legacy stream they run on: whoever uploads
+// ends with this wait.
+void uploads_done() { V2B_CK(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 // first index of a non-finite value in v[0..n), or -1 (host arrays)
 int64_t first_nonfinite(const double *v, int64_t n) {
     for (int64_t i = 0; i < n; i++)
@@ -236,6 +242,7 @@ struct DeviceCg {
         slots = vec<double>(2 * (size_t)nvirtual);
         count = vec<unsigned int>(1);
         V2B_CK(v2b::raise_dynamic_smem(shape.kernel, (int)smem));
+        uploads_done();
     }
     void release() {
         for (void *q : owned) cudaFree(q);
@@ -462,9 +469,7 @@ struct ProjectPlan {
         split_cnt = dalloc<int>(std::max(groups, 1));
         V2B_CK(cudaMemset(split_cnt, 0, std::max(groups, 1) * sizeof(int)));
         for (double *b : {Vt, Us, W, T}) V2B_CK(cudaMemset(b, 0, total * sizeof(double)));
-        // the uploads and fills above ran on the legacy stream, the timed
-        // launches run on a non-blocking one
-        V2B_CK(cudaDeviceSynchronize());
+        uploads_done();
         cudaStream_t s = nullptr;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         V2B_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -480,6 +485,7 @@ struct ProjectPlan {
                 const std::vector<int4> k = split_tiles(d, L, S, g);
                 if (k.empty()) break;
                 V2B_CK(cudaMemcpy(buf, k.data(), k.size() * sizeof(int4), cudaMemcpyHostToDevice));
+                uploads_done();
                 float ms = 0.0f;
                 for (int rep = 0; rep < 4; rep++) {
                     if (rep == 1) V2B_CK(cudaEventRecord(e0, s));
@@ -513,7 +519,7 @@ struct ProjectPlan {
         kstiles = upper.first;
         split_full = full.second;
         split_sym = upper.second;
-        V2B_CK(cudaDeviceSynchronize());   // the chosen lists' uploads complete before any launch
+        V2B_CK(cudaStreamSynchronize(s));   // the timed launches read buf
         cudaFree(buf);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -646,6 +652,7 @@ struct ProjectPlan {
         build_block_jacobi();
         V2B_CK(cudaEventCreateWithFlags(&staged, cudaEventDisableTiming));
         V2B_CK(cudaEventCreateWithFlags(&used, cudaEventDisableTiming));
+        uploads_done();
         fresh = true;
         built = true;
     }
@@ -1429,7 +1436,10 @@ struct v2b_problem {
         if (on && !ev[0])
             for (auto &e : ev) V2B_CK(cudaEventCreate(&e));
         if (level > 1 && !cg_phase) cg_phase = dalloc<unsigned long long>(kCgPhases);
-        if (cg_phase) V2B_CK(cudaMemset(cg_phase, 0, kCgPhases * sizeof(unsigned long long)));
+        if (cg_phase) {
+            V2B_CK(cudaMemset(cg_phase, 0, kCgPhases * sizeof(unsigned long long)));
+            uploads_done();
+        }
         profiling = on;
         phases = level > 1;
         for (int k = 0; k < kClasses; k++) { prof_ms[k] = 0.0; prof_n[k] = 0; }
@@ -1496,6 +1506,7 @@ struct v2b_problem {
         V2B_CK(cudaMemset(stats_counter, 0, 4));
         V2B_CK(cudaMemset(status, 0, 8));
         V2B_CK(cudaMallocHost(&h_readback, 8 * sizeof(double)));
+        uploads_done();
         on_device = true;
     }
 
@@ -1705,6 +1716,7 @@ struct v2b_bpsdp {
             dU = dalloc<double>(np); dx = dalloc<double>(np); dz = dalloc<double>(np);
             status = dalloc<int>(2);
             V2B_CK(cudaMemset(status, 0, 8));
+            uploads_done();
         }
     }
 
@@ -2278,6 +2290,7 @@ int v2b_problem_pack_spatial_density(v2b_problem *p, const double *d_x, double *
             p->ibas_aa_dev = dalloc<int>((size_t)q.n * q.n);
             V2B_CK(cudaMemcpy(p->ibas_aa_dev, q.ibas_aa.data(), sizeof(int) * q.n * q.n,
                               cudaMemcpyHostToDevice));
+            uploads_done();
         }
         v2b::PackArgs a;
         a.n = q.n;

@@ -1,0 +1,156 @@
+"""The library's host code on a CUDA runtime without a GPU (fake_cudart.cpp):
+what it hands to the runtime on first calls and streams.
+
+Each scenario runs in a process of its own, in which the fake takes
+libcudart's place before the library loads."""
+import ctypes
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    from hilbert_b200 import build
+    build.build()
+    d = tmp_path_factory.mktemp("fake")
+    (d / "version").write_text("libcudart.so.12 { global: cuda*; __cuda*; fake_*; local: *; };\n")
+    cuda = os.path.dirname(os.path.dirname(build.nvcc_path()))
+    so = str(d / "libcudart.so.12")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(cuda, "include"),
+                           os.path.join(HERE, "fake_cudart.cpp"), "-o", so, "-Wl,-soname,libcudart.so.12",
+                           f"-Wl,--version-script={d / 'version'}"])
+
+    def run(scenario, *args):
+        out = subprocess.run([sys.executable, os.path.abspath(__file__), so, scenario, *map(str, args)],
+                             capture_output=True, text=True, timeout=600, cwd=ROOT)
+        assert out.returncode == 0, out.stderr[-4000:]
+        return json.loads(out.stdout.strip().splitlines()[-1])
+    return run
+
+
+@pytest.mark.parametrize("call", ["Au", "project", "warm", "mode1", "solve", "profiled", "continued", "bpsdp",
+                                  "pack"])
+def test_uploads_are_waited_for(fake, call):
+    """A pageable cudaMemcpy or a cudaMemset may return before the device holds
+    its result, and nothing orders the legacy stream they run on with a
+    non-blocking one: every table and fill of a problem's first call is waited
+    for before work on another stream can read it."""
+    out = fake("uploads", call)
+    assert out["faults"] == [], out["faults"][:5]
+    assert out["launches"] > 0
+
+
+# ---------------------------------------------------------------- scenarios
+class Host:
+    """The library on the fake runtime; device vectors are numpy arrays."""
+
+    def __init__(self, so):
+        import numpy as np
+        self.np = np
+        self.rt = ctypes.CDLL(so, mode=ctypes.RTLD_GLOBAL)
+        self.rt.fake_events.restype = ctypes.c_char_p
+        self.rt.fake_fail_at.argtypes = [ctypes.c_long]
+        for f in ("fake_allocations", "fake_faults", "fake_live"):
+            getattr(self.rt, f).restype = ctypes.c_long
+        sys.path.insert(0, ROOT)
+        import hilbert_b200 as hb
+        from hilbert_b200 import _capi
+        assert "torch" not in sys.modules   # its libraries want the real runtime
+        self.hb, self.capi = hb, _capi
+        self.lib = _capi.load()
+
+    def stream(self):
+        s = ctypes.c_void_p()
+        self.rt.cudaStreamCreateWithFlags(ctypes.byref(s), 1)
+        return s
+
+    def events(self):
+        return self.rt.fake_events().decode().splitlines()
+
+    def clear(self):
+        self.rt.fake_clear()
+
+    def problem(self, n=3, pos="DQG", doci=False):
+        return (self.hb.DOCIProblem if doci else self.hb.V2RDMProblem)(n, 2, 2 if doci else 1, pos)
+
+    def call(self, what, p, stream):
+        """the entry point's status"""
+        np, lib = self.np, self.lib
+        vec = lambda k: np.zeros(k).ctypes.data_as(ctypes.c_void_p)   # noqa: E731
+        keep = [np.zeros(max(p.n_primal, p.n_dual)) for _ in range(3)]
+        a, b, c = (v.ctypes.data for v in keep)
+        if what == "Au":
+            return max(lib.v2b_problem_Au(p._h, a, b, stream), lib.v2b_problem_ATu(p._h, a, b, stream))
+        if what == "project":
+            return lib.v2b_problem_project(p._h, a, 1.0, b, c, stream)
+        if what == "mode1":
+            lib.v2b_problem_set_projection_mode(p._h, 1)
+            return lib.v2b_problem_project(p._h, a, 1.0, b, c, stream)
+        if what == "warm":
+            return max(lib.v2b_problem_project_warm(p._h, a, 1.0, b, c, stream) for _ in range(2))
+        if what == "pack":
+            g = p.n * (p.n + 1) // 2 if hasattr(p, "n") else 6
+            out = np.zeros(g * (g + 1) // 2 + g)
+            return lib.v2b_problem_pack_spatial_density(p._h, a, out.ctypes.data, out.ctypes.data, stream)
+        if what == "profiled":
+            rc = lib.v2b_problem_set_profiling(p._h, 2)
+            return rc or self.call("solve", p, stream)
+        if what == "continued":
+            rc = self.call("solve", p, stream)
+            return rc or lib.v2b_problem_continue(p._h) or self.call("solve", p, stream)
+        assert what == "solve"
+        o = self.capi.SDPOptions(1e-6, 1e-6, 1e-9, 100, 4)
+        oi, ii, e = ctypes.c_long(), ctypes.c_long(), ctypes.c_double()
+        return lib.v2b_problem_solve(p._h, self.dp(keep[0]), self.dp(keep[1]), self.dp(keep[2]), ctypes.byref(o), 2,
+                                     self.capi.SDP_MONITOR(), 0, None, ctypes.byref(oi), ctypes.byref(ii),
+                                     ctypes.byref(e))
+
+    @staticmethod
+    def dp(v):
+        return v.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+
+    def bpsdp(self, dims):
+        """a host solver whose maps are the identity: its handle and a solve"""
+        np, lib, capi = self.np, self.lib, self.capi
+        n = sum(d * d for d in dims)
+        h = ctypes.c_void_p()
+        o = capi.SDPOptions(1e-6, 1e-6, 1e-9, 3, 4)
+        capi.check(lib.v2b_bpsdp_create(n, n, ctypes.byref(o), ctypes.byref(h)))
+
+        def copy(out, v, _):
+            ctypes.memmove(out, v, 8 * n)
+        cb = capi.SDP_CALLBACK(copy)
+        ones = np.ones(n)
+
+        def solve(dims):
+            x = np.zeros(n)
+            d = (ctypes.c_int * len(dims))(*dims)
+            return lib.v2b_bpsdp_solve(h, self.dp(x), self.dp(ones), self.dp(ones), d, len(dims), 2, cb, cb,
+                                       capi.SDP_MONITOR(), 0, None)
+        return h, solve
+
+
+def uploads(host, call):
+    if call == "bpsdp":
+        h, solve = host.bpsdp([4, 30, 200])
+        rc = solve([4, 30, 200])
+        host.lib.v2b_bpsdp_destroy(h)
+    else:
+        rc = 0
+        for p in (host.problem(), host.problem(5), host.problem(4, doci=True)):
+            rc = max(rc, host.call(call, p, host.stream()))
+            p.close()
+    assert rc in (0, 1), (rc, host.lib.v2b_last_error())
+    ev = host.events()
+    return {"faults": [e for e in ev if e.startswith("FAULT")], "launches": sum(e.startswith("launch") for e in ev)}
+
+
+if __name__ == "__main__":
+    print(json.dumps(globals()[sys.argv[2]](Host(sys.argv[1]), *sys.argv[3:])))

@@ -6,6 +6,12 @@
 
 #include "v2rdm_problem.h"
 
+#ifdef __CUDACC__
+#define V2B_HD __host__ __device__
+#else
+#define V2B_HD
+#endif
+
 namespace v2b {
 
 // The rows of A (dual side) and of A^T (primal side) in SELL-C-sigma form,
@@ -52,6 +58,27 @@ struct CgSide {
 struct CgTables {
     CgSide dual, prim;
 };
+
+// A virtual warp's run of slices b .. e - 1 and where the CG kernel finds its
+// tables in shared memory: entries, then lengths, then slice offsets.
+struct CgRun {
+    uint32_t b, e, gw;   // slices; the virtual warp, 0xffffffff for none
+    uint32_t off;        // word of slice b's offset
+    // word where entry 0 of the side would stand: below 0 for most runs, and
+    // signed, so that base + ent + index is the entry's word as a 64-bit address
+    int32_t ent;
+    uint32_t len;        // byte of slice b's lengths
+};
+// the words of a run's tables
+V2B_HD inline uint32_t cg_table_words(uint32_t nslices, uint32_t nent) {
+    return nent + 8u * nslices + ((nslices + 4u) & ~3u);
+}
+// the run's tables from word `at` on; its entries are e0 .. e0 + ne - 1
+V2B_HD inline void cg_place_run(CgRun &r, uint32_t at, uint32_t e0, uint32_t ne) {
+    r.ent = (int32_t)(at - e0);
+    r.len = 4u * (at + ne);
+    r.off = at + ne + 8u * (r.e - r.b);
+}
 
 // nvirtual virtual CTAs, v of them to a CTA (grid = ceil(nvirtual / v)).  Which
 // CTA hosts a virtual CTA is free, and chosen per side so that the CTAs' work

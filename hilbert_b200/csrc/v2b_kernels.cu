@@ -291,13 +291,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
     __shared__ int fail;
     __shared__ unsigned long long tmark;   // phase clock (CTA 0, thread 0)
     __shared__ uint32_t hostA[V], hostT[V];
-    // per virtual warp and side: first and past-last slice, where the tables
-    // stand in cg_sm (off: word of slice b; ent: word of entry 0; len: byte of
-    // slice b)
-    struct Run {
-        uint32_t b, e, gw, off, ent, len;
-    };
-    __shared__ Run runA[VW], runT[VW];
+    __shared__ CgRun runA[VW], runT[VW];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cta = blockIdx.x;
     if (tid < 16) {
@@ -311,13 +305,13 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
     }
     const uint32_t all = (uint32_t)P.nvirtual * kCgVirtualWarps;
     __syncthreads();
-    auto words = [&](const CgRows &R, const Run &r) {
+    auto words = [&](const CgRows &R, const CgRun &r) {
         return r.gw == 0xffffffffu ? 0u
                                    : cg_table_words(r.e - r.b, (R.off[r.e] & ~kCgPlain) - (R.off[r.b] & ~kCgPlain));
     };
     if (tid < VW) {
-        auto init = [&](Run &r, const CgRows &R, uint32_t vc) {
-            r = Run{0u, 0u, 0xffffffffu, 0u, 0u, 0u};
+        auto init = [&](CgRun &r, const CgRows &R, uint32_t vc) {
+            r = CgRun{0u, 0u, 0xffffffffu, 0u, 0, 0u};
             if (vc == 0xffffffffu) return;
             r.gw = vc * kCgVirtualWarps + tid % kCgVirtualWarps;
             r.b = R.split[r.gw];
@@ -333,29 +327,27 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
         uint32_t at = 0;
         for (int w = 0; w < VW; w++) {
             const uint32_t na = runA[w].off, nt = runT[w].off;
-            runA[w].ent = at;
-            runT[w].ent = SHARED ? at : at + na;
+            runA[w].ent = (int32_t)at;
+            runT[w].ent = (int32_t)(SHARED ? at : at + na);
             at += SHARED ? max(na, nt) : na + nt;
         }
     }
     __syncthreads();
     // start the copy of a run's tables: entries, lengths, offsets
-    auto fetch = [&](const CgRows &R, const Run &r) {
+    auto fetch = [&](const CgRows &R, const CgRun &r) {
         if (r.gw == 0xffffffffu) return;
         const uint32_t e0 = R.off[r.b] & ~kCgPlain, ne = (R.off[r.e] & ~kCgPlain) - e0, n = r.e - r.b;
-        const uint32_t at = r.ent + e0;   // r.ent is the word of entry 0 (below)
+        const uint32_t at = (uint32_t)r.ent + e0;   // the word of entry e0
         for (uint32_t k = 4u * lane; k < ne; k += 128u) cp_async16(cg_sm + at + k, R.ent + e0 + k);
         for (uint32_t k = lane; k < 2u * n; k += 32u)
             cp_async16((uint8_t *)cg_sm + r.len + 16u * k, R.len + 32u * (size_t)r.b + 16u * k);
         for (uint32_t k = lane; k <= n; k += 32u) cp_async4(cg_sm + r.off + k, R.off + r.b + k);
     };
     if (SMEM && tid < VW) {
-        auto place = [&](Run &r, const CgRows &R) {
+        auto place = [&](CgRun &r, const CgRows &R) {
             if (r.gw == 0xffffffffu) return;
-            const uint32_t e0 = R.off[r.b] & ~kCgPlain, ne = (R.off[r.e] & ~kCgPlain) - e0, at = r.ent;
-            r.ent = at - e0;
-            r.len = 4u * (at + ne);
-            r.off = at + ne + 8u * (r.e - r.b);
+            const uint32_t e0 = R.off[r.b] & ~kCgPlain, ne = (R.off[r.e] & ~kCgPlain) - e0;
+            cg_place_run(r, (uint32_t)r.ent, e0, ne);
         };
         place(runA[tid], P.dual);
         place(runT[tid], P.prim);
@@ -413,7 +405,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
     };
     // t = A^T x over a run's slices: stored except at singles, squares into
     // loc in order (loc null: no squares)
-    auto apply_T = [&](const Run &r, const auto &x, double *loc) {
+    auto apply_T = [&](const CgRun &r, const auto &x, double *loc) {
         const uint32_t e = r.e;
         const Words<SMEM> ent{SMEM ? cg_sm + r.ent + lane : P.prim.ent + lane};
         const Words<SMEM> off{SMEM ? cg_sm + r.off - r.b : P.prim.off};
@@ -474,7 +466,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
     // own0(position) is loaded with the entries, self(own) is the p that the
     // row's singles take
     const Operand<false> tx{nullptr, P.t, 0.0};
-    auto apply_A = [&](const Run &r, auto &&own0, auto &&self, auto &&f) {
+    auto apply_A = [&](const CgRun &r, auto &&own0, auto &&self, auto &&f) {
         const uint32_t e = r.e;
         const Words<SMEM> ent{SMEM ? cg_sm + r.ent + lane : P.dual.ent + lane};
         const Words<SMEM> off{SMEM ? cg_sm + r.off - r.b : P.dual.off};
@@ -548,7 +540,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
     auto own_rows = [&](auto &&load, auto &&store) {
 #pragma unroll
         for (int h = 0; h < H; h++) {
-            const Run &r = runA[warp + h * NW];
+            const CgRun &r = runA[warp + h * NW];
             if (r.gw == 0xffffffffu) continue;
             for (uint32_t s = r.b; s < r.e; s += C) {
                 uint32_t o[C];
@@ -579,7 +571,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
         const Operand<false> yx{nullptr, P.yp, 0.0};
 #pragma unroll
         for (int h = 0; h < H; h++) {
-            const Run &r = runT[warp + h * NW];
+            const CgRun &r = runT[warp + h * NW];
             if (r.gw == 0xffffffffu) continue;
             apply_T(r, yx, nullptr);
             long_T(r.gw, yx, nullptr);
@@ -599,7 +591,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
 #pragma unroll
         for (int h = 0; h < H; h++) {
             loc[h] = 0.0;
-            const Run &r = runA[warp + h * NW];
+            const CgRun &r = runA[warp + h * NW];
             if (r.gw == 0xffffffffu) continue;
             auto f = [&](uint32_t j, double av, const Own &o) {
                 const double v = o.acz + P.mu * (o.b - o.ax) - av;
@@ -624,7 +616,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
 #pragma unroll
         for (int h = 0; h < H; h++) {
             loc[h] = 0.0;
-            const Run &r = runT[warp + h * NW];
+            const CgRun &r = runT[warp + h * NW];
             if (r.gw == 0xffffffffu) continue;
             apply_T(r, px, &loc[h]);
             long_T(r.gw, px, &loc[h]);
@@ -647,7 +639,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) cg_kernel(CgParams P) {
 #pragma unroll
         for (int h = 0; h < H; h++) {
             loc[h] = 0.0;
-            const Run &r = runA[warp + h * NW];
+            const CgRun &r = runA[warp + h * NW];
             if (r.gw == 0xffffffffu) continue;
             auto f = [&](uint32_t j, double q, const Own &o) {
                 const double pn = dir(o);

@@ -55,10 +55,6 @@ struct CgShape {
     int threads;
 };
 CgShape cg_shape(int v, CgTablesIn in);
-// shared-memory words of one virtual warp's tables: slices, their entries
-__host__ __device__ inline uint32_t cg_table_words(uint32_t nslices, uint32_t nent) {
-    return nent + 8u * nslices + ((nslices + 4u) & ~3u);
-}
 constexpr size_t kCgStaticSmem = 4096;   // at least the kernel's static shared memory
 
 // Packed rows of A or A^T (CSR) and the list of those longer than

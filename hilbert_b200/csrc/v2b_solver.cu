@@ -73,6 +73,16 @@ T *dalloc(size_t n) {
     return (T *)p;
 }
 
+// frees and forgets device memory, and pinned host memory
+template <class... T>
+void drop(T *&...p) {
+    ((p ? (void)cudaFree(p) : (void)0, p = nullptr), ...);
+}
+template <class... T>
+void drop_pinned(T *&...p) {
+    ((p ? (void)cudaFreeHost(p) : (void)0, p = nullptr), ...);
+}
+
 // cudaMemcpy from pageable memory and cudaMemset may return before the device
 // holds their result, and the library's streams (non-blocking, as the caller's
 // may be) are not ordered with the legacy stream they run on: whoever uploads
@@ -529,6 +539,7 @@ struct ProjectPlan {
     void build(const std::vector<int> &d) {
         dims = d;
         nblk = (int)d.size();
+        nsmall = nbig = max_big = 0;
         h_off.assign(nblk, 0);
         h_roff_small.assign(nblk, -1);
         h_roff_big.assign(nblk, -1);
@@ -660,31 +671,21 @@ struct ProjectPlan {
         if (!built) return;
         for (auto e : pev) cudaEventDestroy(e);
         pev.clear();
+        pev_used = 0;
         if (staged) cudaEventDestroy(staged);
         if (used) cudaEventDestroy(used);
-        used = nullptr;
-        used_pending = false;
-        staged = nullptr;
-        staged_pending = false;
-        for (void *q : {(void *)boff, (void *)rot_off, (void *)bdim, (void *)counters, (void *)tiles, (void *)stiles, (void *)gtiles,
-                        (void *)ktiles, (void *)kstiles, (void *)split_ws, (void *)split_cnt, (void *)gemm_sched, (void *)rot, (void *)Vt, (void *)Vt2, (void *)Us, (void *)W, (void *)T,
-                        (void *)P, (void *)rec_b, (void *)norm_b, (void *)sub_boff, (void *)sub_roff,
-                        (void *)sub_bdim, (void *)bstate, (void *)orth, (void *)bnorm, (void *)norm_part,
-                        (void *)cls_counts, (void *)done_stamp, (void *)Vsave,
-                        (void *)Tsave, (void *)arena, (void *)crec, (void *)cnorm, (void *)Tc,
-                        (void *)Pc, (void *)bj_dev, (void *)bj_on,
-                        (void *)rowbase, (void *)lam, (void *)Qt, (void *)sub32_boff, (void *)sub32_roff,
-                        (void *)sub32_bdim, (void *)T32, (void *)sign_list, (void *)sign_state, (void *)sign_part, (void *)sign_tiles})
-            cudaFree(q);
-        T32 = nullptr;
-        sign_list = sign_state = nullptr;
-        sign_tiles = nullptr;
-        sign_part = nullptr;
+        staged = used = nullptr;
+        staged_pending = used_pending = false;
+        drop(boff, rot_off, bdim, counters, tiles, stiles, gtiles, ktiles, kstiles, split_ws, split_cnt, gemm_sched, rot,
+             Vt, Vt2, Us, W, T, P, rec_b, norm_b, sub_boff, sub_roff, sub_bdim, sub32_boff, sub32_roff, sub32_bdim,
+             bstate, orth, bnorm, norm_part, cls_counts, done_stamp, Vsave, Tsave, arena, crec, cnorm, Tc, Pc, bj_dev,
+             bj_on, rowbase, lam, Qt, T32, sign_list, sign_state, sign_part, sign_tiles);
+        drop_pinned(h_sub, h_bstate_up, h_state, h_edges, h_arena, h_bjon);
+        arena_bytes = 0;
+        crec_slots = 0;
+        cnorm_n = 0;
         sign_small_max = 0;
         sign_large = false;
-        for (void *q : {(void *)h_sub, (void *)h_bstate_up, (void *)h_state, (void *)h_edges,
-                        (void *)h_arena, (void *)h_bjon})
-            if (q) cudaFreeHost(q);
         built = false;
     }
 

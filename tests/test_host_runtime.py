@@ -47,6 +47,14 @@ def test_uploads_are_waited_for(fake, call):
     assert out["launches"] > 0
 
 
+def test_another_set_of_blocks_uses_no_freed_memory(fake):
+    """A host solver may give other block dimensions on its next call: the plan
+    is given back and built again, its grown cluster lists included."""
+    out = fake("rebuilt")
+    assert out["clusters"] >= 2 and out["faults"] == []
+    assert out["left"] == 0   # destroyed: nothing stays allocated
+
+
 # ---------------------------------------------------------------- scenarios
 class Host:
     """The library on the fake runtime; device vectors are numpy arrays."""
@@ -150,6 +158,17 @@ def uploads(host, call):
     assert rc in (0, 1), (rc, host.lib.v2b_last_error())
     ev = host.events()
     return {"faults": [e for e in ev if e.startswith("FAULT")], "launches": sum(e.startswith("launch") for e in ev)}
+
+
+def rebuilt(host):
+    host.rt.fake_refine_script(1)   # warm blocks form a cluster: its lists live in grown memory
+    h, solve = host.bpsdp([30, 40])
+    rc = [solve(d) for d in ([30, 40], [40, 30], [30, 40])]
+    assert max(rc) <= 1, (rc, host.lib.v2b_last_error())
+    host.lib.v2b_bpsdp_destroy(h)
+    ev = host.events()
+    return {"faults": [e for e in ev if e.startswith("FAULT")], "left": host.rt.fake_live(),
+            "clusters": sum("cluster_rows_kernel" in e for e in ev)}
 
 
 if __name__ == "__main__":

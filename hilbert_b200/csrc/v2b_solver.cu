@@ -82,6 +82,18 @@ template <class... T>
 void drop_pinned(T *&...p) {
     ((p ? (void)cudaFreeHost(p) : (void)0, p = nullptr), ...);
 }
+// Device state that is made on first use: `make` either completes or, when one
+// of its steps fails, what it made is given back by `undo` and the next call
+// starts again.
+template <class M, class U>
+void make_whole(M &&make, U &&undo) {
+    try {
+        make();
+    } catch (...) {
+        undo();
+        throw;
+    }
+}
 
 // cudaMemcpy from pageable memory and cudaMemset may return before the device
 // holds their result, and the library's streams (non-blocking, as the caller's
@@ -153,10 +165,7 @@ struct DeviceOp {
         const int64_t g = (nrows + v2b::kSpmvThreads - 1) / v2b::kSpmvThreads;
         return (int)rows().long_blocks + (int)std::max<int64_t>(1, std::min<int64_t>(g, 148 * 16));
     }
-    void release() {
-        for (void *p : {(void *)rp, (void *)ent, (void *)long_rows}) cudaFree(p);
-        rp = ent = long_rows = nullptr;
-    }
+    void release() { drop(rp, ent, long_rows); }
 };
 
 // the CG kernel's tables and vectors on the device (cg_tables.h)
@@ -168,6 +177,7 @@ struct DeviceCg {
     double *yp = nullptr, *t = nullptr, *slots = nullptr;
     unsigned int *count = nullptr;
     int nvirtual = 0, grid = 0;
+    bool built = false;
     size_t smem = 0;
     v2b::CgShape shape{};
 
@@ -253,10 +263,12 @@ struct DeviceCg {
         count = vec<unsigned int>(1);
         V2B_CK(v2b::raise_dynamic_smem(shape.kernel, (int)smem));
         uploads_done();
+        built = true;
     }
     void release() {
         for (void *q : owned) cudaFree(q);
         owned.clear();
+        built = false;
     }
 };
 
@@ -430,7 +442,7 @@ struct ProjectPlan {
     int nsign_tiles = 0;
     double *sign_part = nullptr;
     int nsign_small = 0, sign_small_max = 0;
-    bool sign_large = false;
+    bool sign_large = false, sign_built = false;
     bool fresh = true;
     bool built = false;
     // 0: warm refinement; 1: selective Jacobi on every block, every call;
@@ -480,13 +492,26 @@ struct ProjectPlan {
         V2B_CK(cudaMemset(split_cnt, 0, std::max(groups, 1) * sizeof(int)));
         for (double *b : {Vt, Us, W, T}) V2B_CK(cudaMemset(b, 0, total * sizeof(double)));
         uploads_done();
-        cudaStream_t s = nullptr;
-        cudaEvent_t e0 = nullptr, e1 = nullptr;
-        V2B_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        V2B_CK(cudaEventCreate(&e0));
-        V2B_CK(cudaEventCreate(&e1));
-        int4 *buf = dalloc<int4>(std::max<size_t>(1, (size_t)kGemmMaxSplit * std::max(tl.size(), stl.size())));
-        auto pick = [&](const std::vector<int4> &L, bool sym, int &n_out) {
+        struct Timing {
+            cudaStream_t s = nullptr;
+            cudaEvent_t e0 = nullptr, e1 = nullptr;
+            int4 *buf = nullptr;
+            ~Timing() {
+                if (s) cudaStreamSynchronize(s);   // the timed launches read buf
+                drop(buf);
+                if (e0) cudaEventDestroy(e0);
+                if (e1) cudaEventDestroy(e1);
+                if (s) cudaStreamDestroy(s);
+            }
+        } tm;
+        V2B_CK(cudaStreamCreateWithFlags(&tm.s, cudaStreamNonBlocking));
+        V2B_CK(cudaEventCreate(&tm.e0));
+        V2B_CK(cudaEventCreate(&tm.e1));
+        tm.buf = dalloc<int4>(std::max<size_t>(1, (size_t)kGemmMaxSplit * std::max(tl.size(), stl.size())));
+        const cudaStream_t s = tm.s;
+        const cudaEvent_t e0 = tm.e0, e1 = tm.e1;
+        int4 *const buf = tm.buf;
+        auto pick = [&](const std::vector<int4> &L, bool sym, int4 *&dev, int &n_out) {
             int best_s = 1;
             float best = 0.0f;
             for (int S : {1, 2, kGemmMaxSplit}) {
@@ -519,23 +544,20 @@ struct ProjectPlan {
             int g = 0;
             const std::vector<int4> k = split_tiles(d, L, best_s, g);
             n_out = (int)k.size();
-            int4 *dev = dalloc<int4>(std::max(n_out, 1));
+            dev = dalloc<int4>(std::max(n_out, 1));
             if (n_out) V2B_CK(cudaMemcpy(dev, k.data(), n_out * sizeof(int4), cudaMemcpyHostToDevice));
-            return std::make_pair(dev, best_s);
+            return best_s;
         };
-        auto full = pick(tl, false, nktiles);
-        auto upper = pick(stl, true, nkstiles);
-        ktiles = full.first;
-        kstiles = upper.first;
-        split_full = full.second;
-        split_sym = upper.second;
-        V2B_CK(cudaStreamSynchronize(s));   // the timed launches read buf
-        cudaFree(buf);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        cudaStreamDestroy(s);
+        split_full = pick(tl, false, ktiles, nktiles);
+        split_sym = pick(stl, true, kstiles, nkstiles);
     }
 
+    // for d, unless it is built for d; a failed build leaves nothing behind
+    void ensure(const std::vector<int> &d) {
+        if (built && dims == d) return;
+        release();
+        make_whole([&] { build(d); }, [&] { release(); });
+    }
     void build(const std::vector<int> &d) {
         dims = d;
         nblk = (int)d.size();
@@ -668,7 +690,6 @@ struct ProjectPlan {
         built = true;
     }
     void release() {
-        if (!built) return;
         for (auto e : pev) cudaEventDestroy(e);
         pev.clear();
         pev_used = 0;
@@ -679,14 +700,18 @@ struct ProjectPlan {
         drop(boff, rot_off, bdim, counters, tiles, stiles, gtiles, ktiles, kstiles, split_ws, split_cnt, gemm_sched, rot,
              Vt, Vt2, Us, W, T, P, rec_b, norm_b, sub_boff, sub_roff, sub_bdim, sub32_boff, sub32_roff, sub32_bdim,
              bstate, orth, bnorm, norm_part, cls_counts, done_stamp, Vsave, Tsave, arena, crec, cnorm, Tc, Pc, bj_dev,
-             bj_on, rowbase, lam, Qt, T32, sign_list, sign_state, sign_part, sign_tiles);
+             bj_on, rowbase, lam, Qt, T32);
         drop_pinned(h_sub, h_bstate_up, h_state, h_edges, h_arena, h_bjon);
         arena_bytes = 0;
         crec_slots = 0;
         cnorm_n = 0;
-        sign_small_max = 0;
-        sign_large = false;
+        release_sign();
         built = false;
+    }
+    void release_sign() {
+        drop(sign_list, sign_state, sign_part, sign_tiles);
+        nsign_small = nsign_tiles = sign_small_max = 0;
+        sign_large = sign_built = false;
     }
 
     // sym: the product is symmetric (Vt W with W = Us Vt^T, Vt^T P Vt, Vt Vt^T):
@@ -858,10 +883,8 @@ struct ProjectPlan {
     void ensure_arena(size_t bytes) {
         if (bytes <= arena_bytes) return;
         bytes = std::max(bytes, arena_bytes * 2);
-        if (arena) cudaFree(arena);
-        if (h_arena) cudaFreeHost(h_arena);
-        arena = nullptr;
-        h_arena = nullptr;
+        drop(arena);
+        drop_pinned(h_arena);
         arena_bytes = 0;
         arena = dalloc<unsigned char>(bytes);
         V2B_CK(cudaMallocHost(&h_arena, bytes));
@@ -869,14 +892,14 @@ struct ProjectPlan {
     }
     void ensure_crec(int64_t slots, int nbig_jobs) {
         if (slots > crec_slots) {
-            if (crec) cudaFree(crec);
-            crec = nullptr;
+            drop(crec);
+            crec_slots = 0;
             crec = dalloc<double2>(slots);
             crec_slots = slots;
         }
         if (nbig_jobs > cnorm_n) {
-            if (cnorm) cudaFree(cnorm);
-            cnorm = nullptr;
+            drop(cnorm);
+            cnorm_n = 0;
             cnorm = dalloc<double>((size_t)nbig_jobs * v2b::kBigCluster);
             cnorm_n = nbig_jobs;
         }
@@ -1274,45 +1297,49 @@ struct ProjectPlan {
         }
     }
 
+    // project_once's block lists and scaling scratch
+    void build_sign(cudaStream_t s) {
+        using namespace v2b;
+        std::vector<int> small, state(nblk, 1);
+        for (int b = 0; b < nblk; b++) {
+            if (dims[b] >= 1 && dims[b] <= kSignSmallDim) {
+                small.push_back(b);
+                sign_small_max = std::max(sign_small_max, dims[b]);
+            } else if (dims[b] > kSignSmallDim) {
+                state[b] = 0;
+                sign_large = true;
+            }
+        }
+        // upper tiles, each element computed once and mirrored: the
+        // iteration amplifies an asymmetry
+        std::vector<int4> tl;
+        for (int b = 0; b < nblk; b++) {
+            if (state[b]) continue;
+            const int nt = (dims[b] + gtile - 1) / gtile;
+            for (int i = 0; i < nt; i++)
+                for (int j = i; j < nt; j++) tl.push_back(make_int4(b, i, j, i < j ? 1 : 3));
+        }
+        std::stable_sort(tl.begin(), tl.end(), [&](const int4 &a, const int4 &b) { return dims[a.x] > dims[b.x]; });
+        nsign_tiles = (int)tl.size();
+        sign_tiles = dalloc<int4>(tl.size());
+        if (nsign_tiles)
+            V2B_CK(cudaMemcpyAsync(sign_tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+        nsign_small = (int)small.size();
+        sign_list = dalloc<int>(small.size());
+        sign_state = dalloc<int>(nblk);
+        sign_part = dalloc<double>(2 * (size_t)kSignSplit * nblk);
+        if (nsign_small) V2B_CK(cudaMemcpyAsync(sign_list, small.data(), small.size() * 4, cudaMemcpyHostToDevice, s));
+        V2B_CK(cudaMemcpyAsync(sign_state, state.data(), nblk * 4, cudaMemcpyHostToDevice, s));
+        V2B_CK(cudaStreamSynchronize(s));   // the lists are host temporaries
+        sign_built = true;
+    }
     // A projection from scratch that leaves no basis behind (mode 0): by the
     // matrix sign function (v2b_sign.cu), small blocks in one CTA each, the
     // larger ones through the GEMM tiles.  No host decision, no copy back.
     void project_once(const double *U, double mu, double *x, double *z, cudaStream_t s, long &launches) {
         using namespace v2b;
         if (nblk == 0 || ntiles == 0) return;
-        if (!sign_list) {   // the blocks' classes, once
-            std::vector<int> small, state(nblk, 1);
-            for (int b = 0; b < nblk; b++) {
-                if (dims[b] >= 1 && dims[b] <= kSignSmallDim) {
-                    small.push_back(b);
-                    sign_small_max = std::max(sign_small_max, dims[b]);
-                } else if (dims[b] > kSignSmallDim) {
-                    state[b] = 0;
-                    sign_large = true;
-                }
-            }
-            // upper tiles, each element computed once and mirrored: the
-            // iteration amplifies an asymmetry
-            std::vector<int4> tl;
-            for (int b = 0; b < nblk; b++) {
-                if (state[b]) continue;
-                const int nt = (dims[b] + gtile - 1) / gtile;
-                for (int i = 0; i < nt; i++)
-                    for (int j = i; j < nt; j++) tl.push_back(make_int4(b, i, j, i < j ? 1 : 3));
-            }
-            std::stable_sort(tl.begin(), tl.end(), [&](const int4 &a, const int4 &b) { return dims[a.x] > dims[b.x]; });
-            nsign_tiles = (int)tl.size();
-            sign_tiles = dalloc<int4>(tl.size());
-            if (nsign_tiles)
-                V2B_CK(cudaMemcpyAsync(sign_tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
-            nsign_small = (int)small.size();
-            sign_list = dalloc<int>(small.size());
-            sign_state = dalloc<int>(nblk);
-            sign_part = dalloc<double>(2 * (size_t)kSignSplit * nblk);
-            if (nsign_small) V2B_CK(cudaMemcpyAsync(sign_list, small.data(), small.size() * 4, cudaMemcpyHostToDevice, s));
-            V2B_CK(cudaMemcpyAsync(sign_state, state.data(), nblk * 4, cudaMemcpyHostToDevice, s));
-            V2B_CK(cudaStreamSynchronize(s));   // the lists are host temporaries
-        }
+        if (!sign_built) make_whole([&] { build_sign(s); }, [&] { release_sign(); });
         if (nsign_small) {
             V2B_CK(launch_sign_small(nsign_small, sign_list, sign_small_max, U, boff, bdim, 1.0 / mu, x, z, s));
             launches++;
@@ -1434,8 +1461,9 @@ struct v2b_problem {
     // projection's phases and the CG kernel's own phase clock
     void set_profiling(int level) {
         const bool on = level > 0;
-        if (on && !ev[0])
-            for (auto &e : ev) V2B_CK(cudaEventCreate(&e));
+        if (on)
+            for (auto &e : ev)
+                if (!e) V2B_CK(cudaEventCreate(&e));
         if (level > 1 && !cg_phase) cg_phase = dalloc<unsigned long long>(kCgPhases);
         if (cg_phase) {
             V2B_CK(cudaMemset(cg_phase, 0, kCgPhases * sizeof(unsigned long long)));
@@ -1449,25 +1477,22 @@ struct v2b_problem {
         for (int k = 0; k < ProjectPlan::kPhases; k++) { plan.ph_ms[k] = 0.0; plan.ph_n[k] = 0; }
     }
 
-    ~v2b_problem() {
-        if (!on_device) return;
+    ~v2b_problem() { release(); }
+    void release() {
         A.release();
         AT.release();
         cg.release();
         plan.release();
-        for (double *p : {x, b, c, y, z, Ax, Acz, ATy, U, y1, y2, cg_out, stats,
-                          stats_partials})
-            cudaFree(p);
-        if (cg_phase) cudaFree(cg_phase);
-        if (pack_layout) cudaFree(pack_layout);
-        cudaFree(stats_counter);
-        cudaFree(ibas_aa_dev);
-        cudaFree(status);
-        if (nonfinite) cudaFree(nonfinite);
-        if (h_readback) cudaFreeHost(h_readback);
-        for (auto &e : ev)
+        drop(x, b, c, y, z, Ax, Acz, ATy, U, y1, y2, cg_out, stats, stats_partials, cg_phase, pack_layout,
+             stats_counter, ibas_aa_dev, status, nonfinite);
+        drop_pinned(h_readback);
+        for (auto &e : ev) {
             if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
         if (stream) cudaStreamDestroy(stream);
+        stream = nullptr;
+        on_device = false;
     }
 
     // host operator tables, built once at creation
@@ -1490,6 +1515,9 @@ struct v2b_problem {
     void setup() {
         if (on_device) return;
         ensure_device();
+        make_whole([&] { setup_device(); }, [&] { release(); });
+    }
+    void setup_device() {
         V2B_CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         A.upload(hostA);
         AT.upload(hostAT);
@@ -1511,11 +1539,9 @@ struct v2b_problem {
         on_device = true;
     }
 
-    void ensure_plan() {
-        if (!plan.built) plan.build(prob.dims);
-    }
+    void ensure_plan() { plan.ensure(prob.dims); }
     void ensure_cg() {   // only a solve needs the CG kernel's tables
-        if (!cg.grid) cg.build(hostA, hostAT, sm_count());
+        if (!cg.built) make_whole([&] { cg.build(hostA, hostAT, sm_count()); }, [&] { cg.release(); });
     }
 
     int grid_for(int64_t rows, int threads) const {
@@ -1696,29 +1722,22 @@ struct v2b_bpsdp {
     ProjectPlan plan;
     cudaStream_t stream = nullptr;
     double *dU = nullptr, *dx = nullptr, *dz = nullptr;
-    int *status = nullptr;
     long launches = 0;
 
     ~v2b_bpsdp() {
         if (!stream) return;
         plan.release();
-        cudaFree(dU); cudaFree(dx); cudaFree(dz); cudaFree(status);
+        drop(dU, dx, dz);
         if (stream) cudaStreamDestroy(stream);
     }
 
     void ensure_plan(const std::vector<int> &dims) {
-        if (dims == plan.dims && dU) return;
         int64_t tot = 0;
         for (int d : dims) tot += (int64_t)d * d;
         if (tot != np) throw std::invalid_argument("sum of squared block dimensions != n_primal");
-        plan.release();
-        plan.build(dims);
-        if (!dU) {
-            dU = dalloc<double>(np); dx = dalloc<double>(np); dz = dalloc<double>(np);
-            status = dalloc<int>(2);
-            V2B_CK(cudaMemset(status, 0, 8));
-            uploads_done();
-        }
+        plan.ensure(dims);
+        for (double **p : {&dU, &dx, &dz})
+            if (!*p) *p = dalloc<double>(np);
     }
 
     int solve(double *x, const double *b, const double *c, const std::vector<int> &dims, int maxiter,
@@ -2288,10 +2307,14 @@ int v2b_problem_pack_spatial_density(v2b_problem *p, const double *d_x, double *
         p->setup();
         const v2b::Problem &q = p->prob;
         if (!p->ibas_aa_dev) {
-            p->ibas_aa_dev = dalloc<int>((size_t)q.n * q.n);
-            V2B_CK(cudaMemcpy(p->ibas_aa_dev, q.ibas_aa.data(), sizeof(int) * q.n * q.n,
-                              cudaMemcpyHostToDevice));
-            uploads_done();
+            int *d = dalloc<int>((size_t)q.n * q.n);
+            make_whole(
+                [&] {
+                    V2B_CK(cudaMemcpy(d, q.ibas_aa.data(), sizeof(int) * q.n * q.n, cudaMemcpyHostToDevice));
+                    uploads_done();
+                },
+                [&] { cudaFree(d); });
+            p->ibas_aa_dev = d;
         }
         v2b::PackArgs a;
         a.n = q.n;

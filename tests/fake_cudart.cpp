@@ -59,6 +59,7 @@ cudaError_t release(void *p) {
     }
     freed[it->first] = it->second;   // never handed out again: a later use shows
     live.erase(it);
+    pending = 0;   // a free waits for the device
     return cudaSuccess;
 }
 bool legacy(cudaStream_t s) { return s == nullptr || s == cudaStreamLegacy; }

@@ -55,6 +55,16 @@ def test_another_set_of_blocks_uses_no_freed_memory(fake):
     assert out["left"] == 0   # destroyed: nothing stays allocated
 
 
+@pytest.mark.parametrize("call", ["Au", "project", "warm", "solve", "bpsdp", "pack"])
+def test_a_call_after_a_failed_allocation_starts_again(fake, call):
+    """Whichever allocation of a first call fails, the call returns an error, and
+    the next one makes what is missing: the launches of an undisturbed call, none
+    with a null pointer in the place of a table."""
+    out = fake("retried", call)
+    assert out["tried"] > 10
+    assert out["wrong"] == []
+
+
 # ---------------------------------------------------------------- scenarios
 class Host:
     """The library on the fake runtime; device vectors are numpy arrays."""
@@ -158,6 +168,58 @@ def uploads(host, call):
     assert rc in (0, 1), (rc, host.lib.v2b_last_error())
     ev = host.events()
     return {"faults": [e for e in ev if e.startswith("FAULT")], "launches": sum(e.startswith("launch") for e in ev)}
+
+
+def retried(host, call):
+    host.rt.fake_refine_script(1)
+
+    def attempt(k):
+        """a fresh object whose first call fails at allocation k: the status of
+        that call and of the next, and the next one's launches"""
+        if call == "bpsdp":
+            h, solve = host.bpsdp([4, 30, 200])
+            first = lambda: solve([4, 30, 200])                                # noqa: E731
+            done = lambda: host.lib.v2b_bpsdp_destroy(h)                       # noqa: E731
+        else:
+            p, s = host.problem(6 if call == "project" else 4, doci=call == "pack"), host.stream()
+            first = lambda: host.call(call, p, s)                              # noqa: E731
+            done = lambda: (p.close(), host.rt.cudaStreamDestroy(s))           # noqa: E731
+        host.clear()
+        host.rt.fake_fail_at(k)
+        rc = [first()]
+        count = host.rt.fake_allocations()
+        host.rt.fake_fail_at(-1)
+        faults = host.rt.fake_faults()
+        host.clear()
+        rc.append(first())
+        ev = host.events()
+        done()
+        ev += [e for e in host.events() if e.startswith("FAULT")]
+        return rc, count, faults, {e for e in ev if e.startswith("launch") or e.startswith("FAULT")}, host.rt.fake_live()
+
+    _, count, _, again, left = attempt(-1)
+    # what a first call launches (its autotuner included) and a second one
+    host_first = set()
+    if call != "bpsdp":
+        p, s = host.problem(6 if call == "project" else 4, doci=call == "pack"), host.stream()
+        host.clear()
+        host.call(call, p, s)
+        host_first = {e for e in host.events() if e.startswith("launch")}
+        p.close()
+        host.rt.cudaStreamDestroy(s)
+    else:
+        h, solve = host.bpsdp([4, 30, 200])
+        host.clear()
+        solve([4, 30, 200])
+        host_first = {e for e in host.events() if e.startswith("launch")}
+        host.lib.v2b_bpsdp_destroy(h)
+    known = again | host_first
+    wrong = [] if left == 0 else [f"{left} allocations left"]
+    for k in range(count):
+        rc, _, faults, seen, left = attempt(k)
+        if rc[0] != host.capi.V2B_CUDA_ERROR or rc[1] > 1 or faults or not seen <= known or left:
+            wrong.append([k, rc, faults, sorted(seen - known)[:3], left])
+    return {"tried": count, "wrong": wrong[:5]}
 
 
 def rebuilt(host):

@@ -423,18 +423,23 @@ struct ProjectPlan {
     }
     // A stand-alone projection returns with its kernels still running on the
     // caller's stream; whoever uses the work arrays next on another stream
-    // waits for them.
+    // waits for them.  Streams are told apart by their ids: a destroyed stream's
+    // handle is given out again, and its work may still be running.
     cudaEvent_t used = nullptr;
-    cudaStream_t used_on = nullptr;
+    unsigned long long used_on = 0;
     bool used_pending = false;
+    static unsigned long long stream_id(cudaStream_t s) {
+        unsigned long long id = 0;
+        V2B_CK(cudaStreamGetId(s, &id));
+        return id;
+    }
     void mark_used(cudaStream_t s) {
         V2B_CK(cudaEventRecord(used, s));
-        used_on = s;
+        used_on = stream_id(s);
         used_pending = true;
     }
     void wait_used(cudaStream_t s) {
-        if (!used_pending) return;
-        if (used_on != s) V2B_CK(cudaStreamWaitEvent(s, used, 0));
+        if (used_pending && used_on != stream_id(s)) V2B_CK(cudaStreamWaitEvent(s, used, 0));
     }
     // project_once: its block lists and scaling scratch
     int *sign_list = nullptr, *sign_state = nullptr;

@@ -65,6 +65,17 @@ def test_a_call_after_a_failed_allocation_starts_again(fake, call):
     assert out["wrong"] == []
 
 
+@pytest.mark.parametrize("second", ["project", "warm", "solve"])
+def test_a_new_stream_with_an_old_handle_waits(fake, second):
+    """The work arrays' next user waits for the last one unless it is on the same
+    stream, which a handle alone does not tell: that of a destroyed stream is
+    given out again while its work may still run."""
+    out = fake("reused", second)
+    assert out["same_handle"]
+    assert out["waits"] == 1
+    assert out["waits_on_the_same_stream"] == 0
+
+
 # ---------------------------------------------------------------- scenarios
 class Host:
     """The library on the fake runtime; device vectors are numpy arrays."""
@@ -220,6 +231,24 @@ def retried(host, call):
         if rc[0] != host.capi.V2B_CUDA_ERROR or rc[1] > 1 or faults or not seen <= known or left:
             wrong.append([k, rc, faults, sorted(seen - known)[:3], left])
     return {"tried": count, "wrong": wrong[:5]}
+
+
+def reused(host, second):
+    p, s = host.problem(4), host.stream()
+    assert host.call("project", p, s) == 0
+    host.clear()
+    assert host.call("project", p, s) == 0
+    same = host.events().count("wait")
+    host.rt.cudaStreamDestroy(s)
+    t = host.stream()
+    host.clear()
+    lib, v = host.lib, host.np.zeros(p.n_primal)
+    if second == "warm":   # one call
+        rc = lib.v2b_problem_project_warm(p._h, v.ctypes.data, 1.0, v.ctypes.data, v.ctypes.data, t)
+    else:
+        rc = host.call(second, p, t)
+    assert rc <= 1
+    return {"same_handle": s.value == t.value, "waits": host.events().count("wait"), "waits_on_the_same_stream": same}
 
 
 def rebuilt(host):

@@ -197,4 +197,54 @@ CgTables build_cg_tables(const PackedOperator &A, const PackedOperator &AT, int 
     return t;
 }
 
+CgPlan plan_cg(const PackedOperator &A, const PackedOperator &AT, int sms) {
+    CgPlan p;
+    // Virtual CTAs of 512 threads: a row per thread, three to an SM at most.
+    // They are spread over one CTA per SM; two of them run as one CTA,
+    // without grid barriers.
+    const int64_t want = (std::max(A.nrows, AT.nrows) + 511) / 512;
+    p.nvirtual = (int)std::max<int64_t>(1, std::min<int64_t>(want, 3 * (int64_t)sms));
+    p.v = p.nvirtual <= 2 ? p.nvirtual : (p.nvirtual + sms - 1) / sms;
+    p.tables = build_cg_tables(A, AT, p.nvirtual, p.v);
+    // where the tables go: both passes' in shared memory, in turn in one
+    // region of it, or left in global memory ((20e,20o), 47 us per CG
+    // iteration in one region: 63 streamed)
+    auto words = [&](bool both) {   // of the CTA with most
+        size_t most = 0;
+        for (size_t c = 0; c < p.tables.dual.host.size() / p.v; c++) {
+            size_t sum = 0;
+            for (int w = 0; w < p.v * kCgVirtualWarps; w++) {
+                size_t n[2] = {0, 0};
+                int k = 0;
+                for (const CgSide *s : {&p.tables.dual, &p.tables.prim}) {
+                    const uint32_t vc = s->host[c * p.v + w / kCgVirtualWarps];
+                    if (vc != kNone) {
+                        const size_t gw = (size_t)vc * kCgVirtualWarps + w % kCgVirtualWarps;
+                        n[k] = cg_table_words(s->split[gw + 1] - s->split[gw],
+                                              s->at(s->split[gw + 1]) - s->at(s->split[gw]));
+                    }
+                    k++;
+                }
+                sum += both ? n[0] + n[1] : std::max(n[0], n[1]);
+            }
+            most = std::max(most, sum);
+        }
+        return most;
+    };
+    const size_t room = 227 * 1024 - kCgStaticSmem;
+    p.in = kCgBoth;
+    p.smem = 4 * words(true);
+    if (p.smem > room && p.v == 3) {
+        p.in = kCgOneRegion;
+        p.smem = 4 * words(false);
+    }
+    if (p.smem > room) {
+        p.in = kCgStreamed;
+        p.smem = 0;
+        if (p.v != 1) p.tables = build_cg_tables(A, AT, p.nvirtual, p.v = 1);
+    }
+    p.grid = (p.nvirtual + p.v - 1) / p.v;
+    return p;
+}
+
 }  // namespace v2b

@@ -86,4 +86,16 @@ V2B_HD inline void cg_place_run(CgRun &r, uint32_t at, uint32_t e0, uint32_t ne)
 // entries say (its loads come in dependent rounds), and neighbours are alike.
 CgTables build_cg_tables(const PackedOperator &A, const PackedOperator &AT, int nvirtual, int v);
 
+// Where the CG kernel reads its tables: shared memory, both passes' side by
+// side or in turn in one region, or global memory.
+enum CgTablesIn { kCgBoth, kCgOneRegion, kCgStreamed };
+constexpr size_t kCgStaticSmem = 4096;   // at least the kernel's static shared memory
+struct CgPlan {
+    CgTables tables;
+    int nvirtual, v, grid;
+    CgTablesIn in;
+    size_t smem;   // dynamic shared memory of a CTA
+};
+CgPlan plan_cg(const PackedOperator &A, const PackedOperator &AT, int sms);
+
 }  // namespace v2b

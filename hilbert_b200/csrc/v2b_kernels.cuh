@@ -45,9 +45,6 @@ struct CgParams {
     unsigned long long *phase_ns;   // null, or 4 sums of ns: initial residual, pass 1 (A^T p),
                                     // pass 2 (A t and the update), and a slot left at zero
 };
-// where the CG kernel reads its tables: shared memory, both passes' side by
-// side or in turn in one region, or global memory
-enum CgTablesIn { kCgBoth, kCgOneRegion, kCgStreamed };
 // The CG kernel for v = 1, 2 or 3 virtual CTAs to a CTA, one CTA per SM
 // (kCgStreamed: v = 1, three CTAs per SM), and its thread count
 struct CgShape {
@@ -55,7 +52,6 @@ struct CgShape {
     int threads;
 };
 CgShape cg_shape(int v, CgTablesIn in);
-constexpr size_t kCgStaticSmem = 4096;   // at least the kernel's static shared memory
 
 // Packed rows of A or A^T (CSR) and the list of those longer than
 // kSpmvLongRow, which the first long_blocks CTAs take

@@ -207,58 +207,18 @@ struct DeviceCg {
         return q;
     }
     void build(const v2b::PackedOperator &A, const v2b::PackedOperator &AT, int sms) {
-        // Virtual CTAs of 512 threads: a row per thread, three to an SM at most.
-        // They are spread over one CTA per SM; two of them run as one CTA,
-        // without grid barriers.
-        const int64_t want = (std::max(A.nrows, AT.nrows) + 511) / 512;
-        nvirtual = (int)std::max<int64_t>(1, std::min<int64_t>(want, 3 * (int64_t)sms));
-        int v = nvirtual <= 2 ? nvirtual : (nvirtual + sms - 1) / sms;
-        v2b::CgTables h = v2b::build_cg_tables(A, AT, nvirtual, v);
-        // where the tables go: both passes' in shared memory, in turn in one
-        // region of it, or left in global memory ((20e,20o), 47 us per CG
-        // iteration in one region: 63 streamed)
-        auto words = [&](bool both) {   // of the CTA with most
-            size_t most = 0;
-            for (size_t c = 0; c < h.dual.host.size() / v; c++) {
-                size_t sum = 0;
-                for (int w = 0; w < v * v2b::kCgVirtualWarps; w++) {
-                    size_t n[2] = {0, 0};
-                    int k = 0;
-                    for (const v2b::CgSide *s : {&h.dual, &h.prim}) {
-                        const uint32_t vc = s->host[c * v + w / v2b::kCgVirtualWarps];
-                        if (vc != 0xffffffffu) {
-                            const size_t gw = (size_t)vc * v2b::kCgVirtualWarps + w % v2b::kCgVirtualWarps;
-                            n[k] = v2b::cg_table_words(s->split[gw + 1] - s->split[gw],
-                                                       s->at(s->split[gw + 1]) - s->at(s->split[gw]));
-                        }
-                        k++;
-                    }
-                    sum += both ? n[0] + n[1] : std::max(n[0], n[1]);
-                }
-                most = std::max(most, sum);
-            }
-            return most;
-        };
-        const size_t room = (227 * 1024 - v2b::kCgStaticSmem) / 4;
-        v2b::CgTablesIn in = v2b::kCgBoth;
-        smem = 4 * words(true);
-        if (smem > 4 * room && v == 3) {
-            in = v2b::kCgOneRegion;
-            smem = 4 * words(false);
-        }
-        if (smem > 4 * room) {
-            in = v2b::kCgStreamed;
-            smem = 0;
-            if (v != 1) h = v2b::build_cg_tables(A, AT, nvirtual, v = 1);
-        }
-        grid = (nvirtual + v - 1) / v;
-        shape = v2b::cg_shape(v, in);
-        dual = rows(h.dual);
-        prim = rows(h.prim);
-        orig = put(h.dual.orig);
-        rp = vec<double2>(h.dual.rows());
-        yp = vec<double>(h.dual.rows());
-        t = vec<double>(h.prim.rows());
+        const v2b::CgPlan h = v2b::plan_cg(A, AT, sms);
+        const v2b::CgTables &tab = h.tables;
+        nvirtual = h.nvirtual;
+        grid = h.grid;
+        smem = h.smem;
+        shape = v2b::cg_shape(h.v, h.in);
+        dual = rows(tab.dual);
+        prim = rows(tab.prim);
+        orig = put(tab.dual.orig);
+        rp = vec<double2>(tab.dual.rows());
+        yp = vec<double>(tab.dual.rows());
+        t = vec<double>(tab.prim.rows());
         slots = vec<double>(2 * (size_t)nvirtual);
         count = vec<unsigned int>(1);
         V2B_CK(v2b::raise_dynamic_smem(shape.kernel, (int)smem));

@@ -1,6 +1,6 @@
 // Prints, for the CG tables of one problem, how far each run's words lie from
 // where the kernel looks for them (0 0: every entry, offset and length is
-// found inside its run's own words).
+// found inside its run's own words), then the form that the kernel takes on 148 SMs.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -22,11 +22,9 @@ int main(int argc, char **argv) {
     spec.doci = argc > 5 && !strcmp(argv[5], "doci");
     const Problem p = make_problem(spec);
     const PackedOperator A = build_A(p), AT = build_AT(p);
-    const int sms = 148;
-    const int64_t want = (std::max(A.nrows, AT.nrows) + 511) / 512;
-    const int nv = (int)std::max<int64_t>(1, std::min<int64_t>(want, 3 * sms));
-    const int v = nv <= 2 ? nv : (nv + sms - 1) / sms, grid = (nv + v - 1) / v;
-    const CgTables t = build_cg_tables(A, AT, nv, v);
+    const CgPlan plan = plan_cg(A, AT, 148);
+    const CgTables &t = plan.tables;
+    const int v = plan.v, grid = plan.grid;
     long runs = 0, wrong = 0;
     for (const bool shared : {false, true})
         for (int c = 0; c < grid; c++) {
@@ -57,5 +55,7 @@ int main(int argc, char **argv) {
             }
         }
     printf("%ld runs, %ld wrong\n", runs, wrong);
+    const char *names[] = {"both", "one region", "streamed"};
+    printf("%d per CTA, %s, %zu bytes\n", v, names[plan.in], plan.smem);
     return 0;
 }

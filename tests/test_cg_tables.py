@@ -30,3 +30,15 @@ def test_runs_are_addressed_inside_their_own_words(check, args):
     and in turn."""
     runs, wrong = (int(w.split()[0]) for w in check(*args)[0].split(", "))
     assert runs > 0 and wrong == 0
+
+
+@pytest.mark.parametrize("args,per_cta,form", [((10, 5, 5, 3, "doci"), 2, "both"), ((2, 1, 1, 3), 1, "both"),
+                                               ((9, 5, 4, 3), 2, "both"), ((18, 9, 9, 3), 3, "both"),
+                                               ((19, 10, 9, 3), 3, "one region"), ((20, 10, 10, 3), 3, "one region"),
+                                               ((22, 11, 11, 3), 1, "streamed"), ((10, 5, 5, 4), 1, "streamed")])
+def test_form_of_the_kernel(check, args, per_cta, form):
+    """Which problems take which form of the CG kernel on 148 SMs (227 KB of
+    shared memory each): the tests of each form name their sizes by this."""
+    v, got, nbytes = check(*args)[1].split(", ")
+    assert (int(v.split()[0]), got) == (per_cta, form)
+    assert int(nbytes.split()[0]) <= 227 * 1024 - 4096

@@ -123,7 +123,8 @@ class Host:
             lib.v2b_problem_set_projection_mode(p._h, 1)
             return lib.v2b_problem_project(p._h, a, 1.0, b, c, stream)
         if what == "warm":
-            return max(lib.v2b_problem_project_warm(p._h, a, 1.0, b, c, stream) for _ in range(2))
+            return (lib.v2b_problem_project_warm(p._h, a, 1.0, b, c, stream) or
+                    lib.v2b_problem_project_warm(p._h, a, 1.0, b, c, stream))
         if what == "pack":
             g = p.n * (p.n + 1) // 2 if hasattr(p, "n") else 6
             out = np.zeros(g * (g + 1) // 2 + g)

@@ -99,7 +99,7 @@ def test_repeated_cold_basis_of_general_blocks(cuda_device, n):
 
 
 def test_split_k_gemm_matches_lapack_and_repeats(cuda_device):
-    """Blocks of 306 to 648 rows (n = 18) with their GEMM tiles cut along K and in
+    """Blocks of 324 and 648 rows (n = 18) with their GEMM tiles cut along K and in
     one piece; the parts are summed in a fixed order, so two projections with one
     plan give the same bits."""
     import torch

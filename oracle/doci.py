@@ -11,6 +11,8 @@ import subprocess
 
 import numpy as np
 
+from .maps import ReferenceNotBuilt
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 ORACLE_SO = os.path.join(HERE, "_build", "libdoci_oracle.so")
 REF_SO = os.path.join(HERE, "_ref", "libdoci_ref.so")
@@ -59,7 +61,7 @@ def _lib(kind):
             lib.dco_guess.argtypes = [ctypes.c_void_p, _dp]
         else:
             if not ref_available():
-                raise FileNotFoundError("reference DOCI library not built: run oracle/build_ref.sh")
+                raise ReferenceNotBuilt("reference DOCI library not built: run oracle/build_ref.sh")
             lib = ctypes.CDLL(REF_SO)
             _bind(lib, "doci_ref_")
             lib.doci_ref_create.argtypes = ([ctypes.c_int] * 3 + [ctypes.c_char_p, ctypes.c_int]

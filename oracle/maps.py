@@ -67,6 +67,10 @@ def _oracle_lib():
     return _olib
 
 
+class ReferenceNotBuilt(FileNotFoundError):
+    """hilbert's own compiled code (oracle/_ref) is asked for where it is not built"""
+
+
 def ref_available():
     return os.path.exists(REF_SO)
 
@@ -75,7 +79,7 @@ def _ref_lib():
     global _rlib
     if _rlib is None:
         if not ref_available():
-            raise FileNotFoundError("reference oracle not built: run oracle/build_ref.sh")
+            raise ReferenceNotBuilt("reference oracle not built: run oracle/build_ref.sh")
         lib = ctypes.CDLL(REF_SO)
         lib.v2b_ref_create.restype = ctypes.c_void_p
         lib.v2b_ref_create.argtypes = ([ctypes.c_int] * 3 + [ctypes.c_char_p] + [ctypes.c_int] * 3

@@ -27,7 +27,7 @@ path.
 ``roofline`` is the CG kernel's: algorithmic bytes 8 (2 n_p + 7 n_d) per CG
 iteration over its CUDA-event launch time, against the measured HBM copy
 bandwidth; ``traffic`` is the kernel's DRAM bytes per iteration from one ncu
-capture on the same problem (CG_DRAM_BYTES_PER_ITERATION) times the launch's
+capture on the same problem (CG_DRAM_BYTES_SMEM_TABLES) times the launch's
 iterations.
 
 ``--impl reference`` times the reference's own CPU implementation of the path
@@ -88,12 +88,14 @@ def fp64_reference(workload):
 # available as a fixture.
 DEVICE_COUNTS = {"df20": {"outer_iterations": 4101, "cg_iterations": 127159}}
 # DRAM bytes the CG kernel moves per CG iteration (dram__bytes_read.sum +
-# dram__bytes_write.sum from one ncu capture of a whole launch: 3.60 + 1.86 GB
-# over 142 iterations and the initial residual, on the same df20 problem;
-# `python -m hilbert_b200.synthetic --n 20 --naux 400 --max-outer 1`).  The
-# bench's launches run the same passes over the same vectors, so their traffic
-# is this figure times their iterations.
-CG_DRAM_BYTES_PER_ITERATION = {"df20": 5.46e9 / 143}
+# dram__bytes_write.sum from one ncu capture of a whole launch, 142 iterations
+# and the initial residual, on the same df20 problem;
+# `python -m hilbert_b200.synthetic --n 20 --naux 400 --max-outer 1`): with its
+# tables read through L2 (9.56 + 4.70 GB), and as it is, with them in shared
+# memory (3.60 + 1.86 GB).  The bench's launches run the same passes over the
+# same vectors, so their traffic is the latter times their iterations.
+CG_DRAM_BYTES_PER_ITERATION = {"df20": 14.26e9 / 143}
+CG_DRAM_BYTES_SMEM_TABLES = {"df20": 5.46e9 / 143}
 
 
 def iteration_counts(workload):
@@ -558,10 +560,12 @@ def run_b200(args, w):
     ach = bytes_launch / (ms_cg / n_cg / 1e3) / 1e9
     roof = {"kernel": "cg_kernel", "bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
             "frac": ach / hbm,
-            "traffic": (CG_DRAM_BYTES_PER_ITERATION[args.workload] * (m + 1)
-                        if args.workload in CG_DRAM_BYTES_PER_ITERATION else None),
+            "traffic": (CG_DRAM_BYTES_SMEM_TABLES[args.workload] * (m + 1)
+                        if args.workload in CG_DRAM_BYTES_SMEM_TABLES else None),
+            "traffic_tables_in_l2": (CG_DRAM_BYTES_PER_ITERATION[args.workload] * (m + 1)
+                                     if args.workload in CG_DRAM_BYTES_PER_ITERATION else None),
             "traffic_source": ("ncu DRAM bytes per CG iteration of one captured launch on the same "
-                               "problem, times (m + 1)" if args.workload in CG_DRAM_BYTES_PER_ITERATION
+                               "problem, times (m + 1)" if args.workload in CG_DRAM_BYTES_SMEM_TABLES
                                else None),
             "algorithmic_bytes": "per CG iteration 8 (2 n_p + 7 n_d) vector bytes (index tables "
                                  f"excluded); (m + 1) iterations per launch, m = {m:.1f}",

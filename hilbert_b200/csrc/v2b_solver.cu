@@ -344,8 +344,8 @@ struct ProjectPlan {
     long refine_large_clusters = 0;   // clusters diagonalised by the Jacobi kernels
     long fb_edges = 0, fb_passes = 0;  // why refined blocks went to Jacobi
     // optional CUDA-event timing of the projection's phases (with the
-    // problem's profiling): 0 GEMM tiles, 1 acceptance test (norms, test,
-    // P), 2 clusters + Newton step, 3 block-Jacobi sweeps, 4 Jacobi kernels
+    // problem's profiling): 0 GEMM tiles (the sign iteration's small blocks
+    // too), 1 acceptance test (norms, test, P), 2 clusters + Newton step, 3 block-Jacobi sweeps, 4 Jacobi kernels
     static constexpr int kPhases = 5;
     bool prof = false;
     std::vector<cudaEvent_t> pev;
@@ -1305,8 +1305,14 @@ struct ProjectPlan {
         using namespace v2b;
         if (nblk == 0 || ntiles == 0) return;
         if (!sign_built) make_whole([&] { build_sign(s); }, [&] { release_sign(); });
+        // a captured call's events could not be read
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (prof) V2B_CK(cudaStreamIsCapturing(s, &capture));
+        const bool timed = capture == cudaStreamCaptureStatusNone;
         if (nsign_small) {
+            if (timed) ph_begin(0, s);
             V2B_CK(launch_sign_small(nsign_small, sign_list, sign_small_max, U, boff, bdim, 1.0 / mu, x, z, s));
+            if (timed) ph_end(s);
             launches++;
         }
         if (!sign_large) return;
@@ -1314,12 +1320,16 @@ struct ProjectPlan {
         const int n = sign_steps(step);
         symmetrize_kernel<<<ntiles, 256, 0, s>>>(U, Us, tiles, boff, bdim);
         V2B_CK(cudaGetLastError());
+        if (timed) ph_begin(1, s);
         V2B_CK(launch_sign_scale(nblk, ntiles, tiles, sign_state, Us, boff, bdim, sign_part, T, s));
+        if (timed) ph_end(s);
         launches += 4;
         auto product = [&](GemmVariant v, const double *A, const double *B, double *C, const double *Cin, double a,
                            double b) {
+            if (timed) ph_begin(0, s);
             V2B_CK(launch_gemm_tiles(v, nsign_tiles, s, A, B, C, sign_tiles, boff, bdim, Cin, Us, a, x, z, nullptr,
                                      orth, gemm_sched, nullptr, nullptr, gtile, b));
+            if (timed) ph_end(s);
             launches++;
         };
         double *X = T, *X2 = P;

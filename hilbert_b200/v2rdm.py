@@ -474,7 +474,9 @@ class V2RDMProblem:
                      "fallback_edges", "fallback_passes", "block_jacobi_sweeps", "fp32_eigensolves")
 
     def refine_counts(self):
-        """counts of the warm eigen-refinement, keyed by REFINE_COUNTS"""
+        """counts of the warm eigen-refinement, keyed by REFINE_COUNTS (a
+        stand-alone projection in mode "refine" has none: it goes by the matrix
+        sign function)"""
         v = (ctypes.c_long * len(self.REFINE_COUNTS))()
         check(self._lib.v2b_problem_refine_counts(self._h, v, len(v)))
         return dict(zip(self.REFINE_COUNTS, v))

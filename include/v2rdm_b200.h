@@ -244,7 +244,10 @@ long v2b_problem_kernel_launches(const v2b_problem *p);
 int v2b_problem_set_profiling(v2b_problem *p, int on);
 /* with profiling level 2: CUDA-event time of the projection's phases, the first
  * count of: [0] GEMM tiles, [1] acceptance test, [2] clusters + Newton step,
- * [3] block-Jacobi sweeps, [4] Jacobi kernels (no reference counterpart) */
+ * [3] block-Jacobi sweeps, [4] Jacobi kernels (no reference counterpart).  A
+ * stand-alone projection (v2b_problem_project, mode 0) counts its products and
+ * its small blocks' kernel in [0], its norms in [1]; calls between solves are
+ * added by the next solve, captured ones are not timed. */
 int v2b_problem_projection_profile(const v2b_problem *p, double *ms, long *n, int count);
 /* with profiling level 2: milliseconds of the CG kernel's phases, barrier to
  * barrier on the kernel's own clock, the first count of: [0] initial
@@ -266,7 +269,8 @@ int v2b_problem_projection_counts(const v2b_problem *p, long *calls, long *rotat
  * block-Jacobi sweeps for a cluster above 64 rows, [5] ... for too many
  * non-separable pairs, [6] blocks handed to the Jacobi kernels after their
  * passes or sweeps ran out, [7] block-Jacobi sweeps run, [8] FP32
- * eigensolves of blocks (projection mode 2). */
+ * eigensolves of blocks (projection mode 2).  A stand-alone projection in mode
+ * 0 goes by the matrix sign function and adds to none of them. */
 int v2b_problem_refine_counts(const v2b_problem *p, long *counts, int n);
 /* No counterpart in the reference.  Projection method of the device solve:
  * 0 (default) warm refinement with block-Jacobi and Jacobi fallbacks; 1 the

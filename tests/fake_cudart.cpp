@@ -27,6 +27,7 @@ cudaError_t last = cudaSuccess;
 
 struct Stream {
     unsigned long long id;
+    bool capturing;
 };
 std::vector<Stream *> spare;   // destroyed streams: their handles are given out again
 unsigned long long next_id = 10;
@@ -133,6 +134,7 @@ void fake_clear() {
     faults = 0;
 }
 void fake_refine_script(int k) { refine_script = k; }
+void fake_capture(cudaStream_t s, int on) { ((Stream *)s)->capturing = on; }
 
 // ------------------------------------------------ memory
 cudaError_t cudaMalloc(void **p, size_t n) { return allocate(p, n); }
@@ -173,7 +175,7 @@ cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st) {
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
     Stream *p = spare.empty() ? new Stream : spare.back();
     if (!spare.empty()) spare.pop_back();
-    *p = Stream{next_id++};
+    *p = Stream{next_id++, false};
     *s = (cudaStream_t)p;
     live_streams++;
     return cudaSuccess;
@@ -185,6 +187,10 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
 }
 cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long *id) {
     *id = legacy(s) ? 1 : ((Stream *)s)->id;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus *st) {
+    *st = !legacy(s) && ((Stream *)s)->capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {

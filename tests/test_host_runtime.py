@@ -76,6 +76,15 @@ def test_a_new_stream_with_an_old_handle_waits(fake, second):
     assert out["waits_on_the_same_stream"] == 0
 
 
+def test_stand_alone_projections_are_profiled(fake):
+    """Profiling level 2 times a stand-alone projection's launches beside the
+    solver's (collected by the next solve), but not inside a capture."""
+    out = fake("profiled_projection")
+    gemm, acceptance = out["project"][0] - out["none"][0], out["project"][1] - out["none"][1]
+    assert gemm == out["launched"] and acceptance == 1
+    assert out["captured"] == out["none"]
+
+
 # ---------------------------------------------------------------- scenarios
 class Host:
     """The library on the fake runtime; device vectors are numpy arrays."""
@@ -250,6 +259,28 @@ def reused(host, second):
         rc = host.call(second, p, t)
     assert rc <= 1
     return {"same_handle": s.value == t.value, "waits": host.events().count("wait"), "waits_on_the_same_stream": same}
+
+
+def profiled_projection(host):
+    out = {}
+    for what in ("none", "project", "captured"):
+        p, s = host.problem(6), host.stream()
+        assert host.lib.v2b_problem_set_profiling(p._h, 2) == 0
+        assert host.call("project", p, s) == 0        # builds the plan and its lists
+        assert host.lib.v2b_problem_set_profiling(p._h, 2) == 0
+        host.clear()
+        host.rt.fake_capture(s, what == "captured")
+        if what != "none":
+            assert host.call("project", p, s) == 0
+        host.rt.fake_capture(s, False)
+        if what == "project":   # the small blocks' kernel and the tiles
+            out["launched"] = sum("gemm_tiles" in e or "sign_small" in e for e in host.events())
+        assert host.call("solve", p, s) <= 1
+        ms, n = (ctypes.c_double * 5)(), (ctypes.c_long * 5)()
+        assert host.lib.v2b_problem_projection_profile(p._h, ms, n, 5) == 0
+        out[what] = list(n)
+        p.close()
+    return out
 
 
 def rebuilt(host):

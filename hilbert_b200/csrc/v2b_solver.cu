@@ -345,7 +345,8 @@ struct ProjectPlan {
     long fb_edges = 0, fb_passes = 0;  // why refined blocks went to Jacobi
     // optional CUDA-event timing of the projection's phases (with the
     // problem's profiling): 0 GEMM tiles (the sign iteration's small blocks
-    // too), 1 acceptance test (norms, test, P), 2 clusters + Newton step, 3 block-Jacobi sweeps, 4 Jacobi kernels
+    // too), 1 acceptance test (norms, test, P), 2 clusters + Newton step,
+    // 3 block-Jacobi sweeps, 4 Jacobi kernels
     static constexpr int kPhases = 5;
     bool prof = false;
     std::vector<cudaEvent_t> pev;

@@ -384,23 +384,36 @@ struct ProjectPlan {
     }
     // A stand-alone projection returns with its kernels still running on the
     // caller's stream; whoever uses the work arrays next on another stream
-    // waits for them.  Streams are told apart by their ids: a destroyed stream's
-    // handle is given out again, and its work may still be running.
+    // waits for them.  A handle alone does not tell streams apart: a destroyed
+    // stream's is given out again, and its work may still be running.  A stream
+    // under capture has no id to ask for (0 here); it is known by its handle.
     cudaEvent_t used = nullptr;
-    unsigned long long used_on = 0;
+    cudaStream_t used_on = nullptr;
+    unsigned long long used_id = 0;
     bool used_pending = false;
+    static bool capturing(cudaStream_t s) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        V2B_CK(cudaStreamIsCapturing(s, &st));
+        return st != cudaStreamCaptureStatusNone;
+    }
     static unsigned long long stream_id(cudaStream_t s) {
         unsigned long long id = 0;
-        V2B_CK(cudaStreamGetId(s, &id));
+        if (!capturing(s)) V2B_CK(cudaStreamGetId(s, &id));
         return id;
     }
     void mark_used(cudaStream_t s) {
         V2B_CK(cudaEventRecord(used, s));
-        used_on = stream_id(s);
+        used_on = s;
+        used_id = stream_id(s);
         used_pending = true;
     }
     void wait_used(cudaStream_t s) {
-        if (used_pending && used_on != stream_id(s)) V2B_CK(cudaStreamWaitEvent(s, used, 0));
+        if (!used_pending) return;
+        if (used_on == s) {
+            const unsigned long long id = stream_id(s);
+            if (id == used_id || id == 0 || used_id == 0) return;
+        }
+        V2B_CK(cudaStreamWaitEvent(s, used, 0));
     }
     // project_once: its block lists and scaling scratch
     int *sign_list = nullptr, *sign_state = nullptr;
@@ -1307,9 +1320,7 @@ struct ProjectPlan {
         if (nblk == 0 || ntiles == 0) return;
         if (!sign_built) make_whole([&] { build_sign(s); }, [&] { release_sign(); });
         // a captured call's events could not be read
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (prof) V2B_CK(cudaStreamIsCapturing(s, &capture));
-        const bool timed = capture == cudaStreamCaptureStatusNone;
+        const bool timed = prof && !capturing(s);
         if (nsign_small) {
             if (timed) ph_begin(0, s);
             V2B_CK(launch_sign_small(nsign_small, sign_list, sign_small_max, U, boff, bdim, 1.0 / mu, x, z, s));

@@ -186,6 +186,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
     return cudaSuccess;
 }
 cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long *id) {
+    if (!legacy(s) && ((Stream *)s)->capturing) return cudaErrorStreamCaptureUnsupported;
     *id = legacy(s) ? 1 : ((Stream *)s)->id;
     return cudaSuccess;
 }

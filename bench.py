@@ -85,7 +85,8 @@ def fp64_reference(workload):
 # Outer and CG iteration counts of the device's own FP64 solve of each
 # workload to convergence (default path, B200): what the CPU arm's sampled
 # per-iteration costs are scaled by when the CPU oracle's full solve is not
-# available as a fixture.
+# available as a fixture (the GEMM split's other choices give 127,006 CG
+# iterations).
 DEVICE_COUNTS = {"df20": {"outer_iterations": 4101, "cg_iterations": 127159}}
 # DRAM bytes the CG kernel moves per CG iteration (dram__bytes_read.sum +
 # dram__bytes_write.sum from one ncu capture of a whole launch, 142 iterations

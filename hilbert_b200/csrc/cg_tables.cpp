@@ -206,9 +206,15 @@ CgPlan plan_cg(const PackedOperator &A, const PackedOperator &AT, int sms) {
     p.nvirtual = (int)std::max<int64_t>(1, std::min<int64_t>(want, 3 * (int64_t)sms));
     p.v = p.nvirtual <= 2 ? p.nvirtual : (p.nvirtual + sms - 1) / sms;
     p.tables = build_cg_tables(A, AT, p.nvirtual, p.v);
-    // where the tables go: both passes' in shared memory, in turn in one
-    // region of it, or left in global memory ((20e,20o), 47 us per CG
-    // iteration in one region: 63 streamed)
+    // Where the tables go: both passes' in shared memory if they fit, else in
+    // turn in one region of it, else left in global memory.  us per CG iteration
+    // with both / one region / streamed: 9 orbitals 12.0 / 11.9 / 16.8, 14: 16.0 /
+    // 18.9 / 29.5, 16: 21.2 / 23.9 / 38.0, 8 with T2 23.7 / 26.5 / 31.1; 18, where
+    // both just fit, 38.9 / 32.7 / 55.9 (the one size measured where one region
+    // was the better).  Where both do not fit, one region / streamed: 19 orbitals
+    // 65.1 / 71.8, 20: 48.3 / 64.8, 9 with T2 51.6 / 55.6.  Where neither fits,
+    // streamed against the former kernel: 22 orbitals 95 (134), 24: 133 (195), 10
+    // with T2 112 (177).
     auto words = [&](bool both) {   // of the CTA with most
         size_t most = 0;
         for (size_t c = 0; c < p.tables.dual.host.size() / p.v; c++) {

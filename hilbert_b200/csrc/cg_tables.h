@@ -23,10 +23,10 @@ namespace v2b {
 // are positions of the other side, so a row's own values are read and written
 // without an index.
 //   entry: bits 0..26 position, 27..30 palette index, 31 group flag
-//   len:   bits 0..5 entries of the row (0xff on padding), bit 7 kCgSingle
-// A primal variable with one entry in A^T and one in A (a Q2, G2, T2, ...
-// element in its own defining row: 84% of the (20e,20o) DQG variables) is a
-// "single": its constraint forms t = coef * p from its own p, the entry
+//   len:   bits 0..5 entries of the row (kCgPadding on padding), bit 7 kCgSingle
+// A primal variable with one entry in A^T and one in A, of the same coefficient
+// (a Q2, G2, T2, ... element in its own defining row: 84% of the (20e,20o) DQG
+// variables), is a "single": its constraint forms t = coef * p from its own p, the entry
 // (position kCgSelf) needs no gather, and t is not stored.
 //
 // split[w] .. split[w + 1] - 1 are the slices of virtual warp w, long rows

@@ -9,8 +9,8 @@
 //   Y  = Vt^T P               gemm<T,N>
 //   U+ = Y Vt                 gemm<N,N> with the projection epilogue
 //                             x = U+ / mu,  z = U+ - sym(U)
-// Every gemm launch covers all blocks of the problem: the grid is the list of
-// 64 x 64 output tiles of every block.
+// Every gemm launch covers all blocks of the problem: its work is the list of
+// output tiles (64 x 64 or 32 x 32) of every block.
 #include "v2b_eig.cuh"
 #include "v2b_kernels.cuh"
 
@@ -25,8 +25,9 @@ namespace v2b {
 //
 // FP64 tensor cores (mma.sync m8n8k4 .f64): a 64 x 64 output tile per CTA of
 // 4 warps, each warp a 32 x 32 sub-tile of 4 x 4 m8n8 fragments (32
-// accumulators per thread).  K runs in chunks of 16 through a cp.async
-// pipeline of three stages (8-byte copies: a block of odd dimension starts at an
+// accumulators per thread); a 32 x 32 tile has a quarter of each.  K runs in
+// chunks of 16 through a cp.async pipeline of three stages, six for the smaller
+// tile (8-byte copies: a block of odd dimension starts at an
 // odd double, so 16-byte alignment is not available; out-of-range elements
 // are zero-filled by the copy itself).  Each operand tile is stored with its
 // global contiguous index innermost (k-major when the matrix is read down
@@ -48,7 +49,10 @@ namespace v2b {
 //
 // Tile size: 64 x 64 tiles reuse their operands twice as often, 32 x 32 tiles
 // (a quarter of the work, 0.14 us of MMAs per K chunk against 0.54) give four
-// times as many CTAs and finish sooner where 64 x 64 tiles leave SMs idle.
+// times as many CTAs and finish sooner where 64 x 64 tiles leave SMs idle.  A
+// warm projection pair and a stand-alone projection, us with 32 / 64: 6 orbitals
+// 418 / 552 and 857 / 1,650, 9: 649 / 943 and 1,026 / 2,056, 11: 744 / 1,091 and
+// 1,224 / 2,534, 5 with T2: 568 / 999 and 1,060 / 2,126.
 constexpr int kGemmBK = 16;
 constexpr int kGemmThreads = 128;
 constexpr int kPadK = kGemmBK + 4;      // m-major rows: 16 + 4 doubles

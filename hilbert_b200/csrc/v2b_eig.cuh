@@ -27,7 +27,9 @@ constexpr int kGemmMaxSplit = 4;   // K parts of one output tile at most
 
 // Host launcher of gemm_tiles_kernel<TA, TB, EPI> (defined, with the kernel
 // instantiations, in v2b_eig.cu).  variant: 0 <N,T,store>, 1 <N,N,store>,
-// 2 <T,N,store>, 3 <N,N,project>, 4 <N,N,add>, 5 <N,T,Newton-Schulz>.
+// 2 <T,N,store>, 3 <N,N,project>, 4 <N,N,add>, 5 <N,T,Newton-Schulz>,
+// 6 <N,T,linear>, 7 <N,T,sign>.  inv_mu is 1 / mu in the variants that write x
+// and z (3, 7) and the weight of Cin in 6, beta the weight of the product there.
 // With bstate non-null, tiles of blocks whose state is not 0 (refinement in
 // progress) are skipped.  sched: two ints, zero before the first launch, that
 // make the grid persistent (tiles taken in list order; the kernel leaves them

@@ -98,7 +98,7 @@ __device__ __forceinline__ double block_norm(const double *part, int blk) {
 // counted and non-separable ones recorded as edges; the last CTA of a block to
 // finish sets its state (done -> done_stamp = stamp, for write_p_kernel).
 // (20e,20o), all blocks: 24 us; with columns read from memory by 16 CTAs a
-// block 72.
+// block 63.
 __global__ void __launch_bounds__(kRefineThreads)
     refine_classify_kernel(const double *__restrict__ T, const int64_t *__restrict__ boff,
                            const int *__restrict__ bdim, int *__restrict__ bstate,

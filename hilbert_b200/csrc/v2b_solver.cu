@@ -273,7 +273,10 @@ struct ProjectPlan {
     int nktiles = 0, nkstiles = 0;
     // The GEMMs' tile size.  32 where the 64 x 64 tiles would leave SMs idle,
     // if no block has tiles to cut along K: 9.1 us a launch against 22.6 for
-    // the blocks of 45 to 200 rows of (10e,10o).
+    // the blocks of 45 to 200 rows of (10e,10o) (other sizes in v2b_eig.cu).  The
+    // line is where the tiles cut along K begin, not where 64 becomes the better:
+    // past it 32 was still faster, a warm pair 785 us against 1,116 at (12e,12o)
+    // and 1,223 against 1,646 at (16e,16o).
     int gtile = v2b::kGemmTile;
     int4 *gtiles = nullptr;   // the full list in that size (the elementwise kernels keep 64)
     int ngtiles = 0;
@@ -1427,7 +1430,8 @@ struct v2b_problem {
     cudaEvent_t ev[2 * kClasses] = {};
     double prof_ms[kClasses] = {};
     long prof_n[kClasses] = {};
-    // CG phases, summed by the kernel's own clock: initial residual, A^T p, A t, update
+    // CG phases, summed by the kernel's own clock: initial residual, A^T p, A t
+    // with the update, and one of the C ABI that stays zero
     static constexpr int kCgPhases = 4;
     unsigned long long *cg_phase = nullptr;
     bool phases = false;   // profiling level 2
